@@ -744,6 +744,7 @@ int fe_form_bind_sparsity(fe_form f, fe_sparsity s, void* stream) {
     try {
       launch_build_slotmap(*f, st);
       check_device_errors(f->ctx, st, FE_ERR_PATTERN);
+      if (rows_default(*f)) build_rows_plan(*f, st);
     } catch (...) {
       f->sp = nullptr;  // the byte map is incomplete: the form stays unbound
       throw;
@@ -977,6 +978,18 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
                             a->mesh->num_cells >= (int64_t(1) << 20);
     const bool want_block = (flags & FE_ASM_BLOCK) || auto_block;
     if (flags & FE_ASM_BLOCK) FE_REQUIRE(block_supported(*a), "the block variant supports P1/P2 stiffness only");
+    // the row walk wherever the form has its plan (built when the pattern was
+    // bound) and no other variant is asked for
+    if (flags & FE_ASM_ROW_WALK) {
+      if (!a->rows_plan && !view) build_rows_plan(*a, st);
+      FE_REQUIRE(!view && rows_supported(*a, bc0, bc1, st),
+                 "the row walk supports FP64 P1/P2 stiffness with one space and one set of BCs, on conforming cells");
+    }
+    if (!(flags & (FE_ASM_ATOMIC | FE_ASM_FULL_SCATTER | FE_ASM_BLOCK | FE_ASM_COALESCED | FE_ASM_GROUPED)) && !view &&
+        rows_supported(*a, bc0, bc1, st)) {
+      assemble_matrix_rows(*a, values, bc0, diagonal, zero, st);
+      return;
+    }
     if (want_block && block_supported(*a)) {
       assemble_matrix_block(*a, values, bc0, bc1, zero, diagonal, st);
       return;

@@ -155,6 +155,12 @@ struct fe_bc_s {
     int64_t chunk = 0, grid = 0;
   };
   mutable std::map<uint64_t, std::unique_ptr<DiagSlots>> diag_slots;  // a cache: filled on const use
+  // per pattern id, what this BC touches (fe_rows.cu); built on first use
+  struct RowFlags {
+    fe::DevBuf<uint8_t> flags;   // per row: bit 0 a BC row, bit 1 a row with a BC column
+    fe::DevBuf<uint32_t> mask;   // bit s: the column of slot s is a BC column
+  };
+  mutable std::map<uint64_t, std::unique_ptr<RowFlags>> row_flags;
   fe::DevBuf<uint8_t> markers;   // [num_dofs]
   fe::DevBuf<int32_t> dofs;      // [n_bc], owned first
   fe::DevBuf<double> g;          // [num_dofs]
@@ -219,6 +225,11 @@ struct fe_form_s {
   struct GroupPlan;
   std::unique_ptr<GroupPlan> groups;
 
+  // row-walk plan (fe_rows.cu); built when the pattern is bound, null where
+  // the walk does not apply
+  struct RowsPlan;
+  std::unique_ptr<RowsPlan> rows_plan;
+
   bool group_plan_failed = false;  // the mesh has no repeated group structure
   fe_form_s();
   ~fe_form_s();
@@ -282,6 +293,26 @@ struct fe_form_s::TilePlan {
 struct fe_form_s::RowPlan {
   fe::DevBuf<int32_t> inc_ptr;        // [block rows + 1]
   fe::DevBuf<int32_t> inc;            // incidences cell*k + i, grouped by row
+};
+
+struct fe_form_s::RowsPlan {
+  // rows of one kind (vertex, edge node, face node) in groups of 32, one group a warp;
+  // record (step, lane) of a group stands at (steps[group] + step) * 32 + lane
+  struct Part {
+    int64_t ngroups = 0;
+    int parts = 1;                    // vertex rows: warps that share a group's cells
+    int stride = 0;                   // doubles of a row's segment in shared memory (odd)
+    bool gaps = false;                // some rows have slots that no cell adds to
+    fe::DevBuf<int4> own;             // [groups*32] row (-1: none), its vertices, the slots of its own columns
+    fe::DevBuf<int32_t> steps;        // [groups+1] prefix sums of the groups' longest walks
+    fe::DevBuf<uint4> rec;            // records: vertices with marks, slot bytes
+    fe::DevBuf<uint2> rec1;           // P1 records
+    fe::DevBuf<int32_t> cell;         // cell of each record
+  };
+  Part part[3];
+  fe::DevBuf<double4> x4;             // vertex coordinates, 32 bytes apart
+  uint64_t map_id = 0;                // P1 coefficient dofmap last compared with the mesh's vertices
+  bool map_same = false;
 };
 
 struct fe_form_s::BlockPlan {
@@ -518,6 +549,16 @@ void reset_batch_plan(fe_form_s& f);
 void assemble_matrix_batch(fe_form_s& f, int num_instances, const double* const* coefficients,
                            double* const* values, const fe_bc_s* bc0, const fe_bc_s* bc1, double diagonal,
                            bool zero, cudaStream_t s);
+
+// row-walk assembly (fe_rows.cu): where it is the default (rows_default) the
+// plan is built with the slot map; build_rows_plan leaves none where the walk
+// does not apply
+bool rows_default(const fe_form_s& f);
+void build_rows_plan(fe_form_s& f, cudaStream_t s);
+void reset_rows_plan(fe_form_s& f);
+bool rows_supported(fe_form_s& f, const fe_bc_s* bc0, const fe_bc_s* bc1, cudaStream_t s);
+void assemble_matrix_rows(fe_form_s& f, double* values, const fe_bc_s* bc, double diagonal, bool zero,
+                          cudaStream_t s);
 
 // row-gather assembly (fe_rowgather.cu) for P1 stiffness
 bool rowgather_supported(const fe_form_s& f);

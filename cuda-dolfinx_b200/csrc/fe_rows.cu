@@ -1,0 +1,1365 @@
+// Row-walk matrix assembly: one thread owns one CSR row (the default for the
+// cell stiffness forms).
+//
+// The scatter kernels (fe_kernels.cu) send every element entry to the L2 as
+// an FP64 reduction (531 M of them for 205 M nonzeros at P2 n=96) into values
+// a zero pass has cleared before; the L2's reduction rate bounds them at any
+// occupancy.  Here a thread walks the cells around its row's node instead,
+// adds their entries into the row's segment in shared memory, where nothing
+// else writes (no atomics, a fixed order: the result is bitwise
+// reproducible), and the warp then stores its 32 rows once, coalesced.  There
+// is no zero pass and no reduction, and only row i of an element tensor is
+// evaluated for row i.
+//
+// What makes the walk cheap is its plan (built with the slot map when a form
+// binds its pattern): the rows of a warp are of one kind (vertex, edge node,
+// face node) and of nearly one length, so their code does not diverge; every
+// cell is listed with its vertices in the row's own order (its vertex, or its
+// edge's or face's vertices, first), so that an entry's formula is fixed at
+// compile time; the cells follow one another through their common faces
+// (around an edge; around a vertex as strips of the triangles opposite it), so
+// that a step fetches one new vertex and keeps the others in registers; and
+// the slot bytes of a step's columns stand in the same record.
+//
+// Element entries, with n_x the gradient of barycentric coordinate x times
+// det J, w = k / |det J| and xy = n_x . n_y (for affine cells grad lambda_x .
+// grad lambda_y |det J| = xy / |det J|): integrals of products of barycentric
+// coordinates are exact rationals, so row i is a few products of the xy.
+//
+// Reference counterpart: assemble_<I>_c_mat (CUDAFormIntegral.cpp:1103-1226)
+// with its zero and set_diagonal passes (CUDAAssembler.cpp:38-164).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cub/cub.cuh>
+#include <memory>
+
+#include "fe_internal.h"
+
+namespace fe {
+namespace {
+
+constexpr unsigned kAll = 0xffffffffu;
+constexpr int kMaxStar = 128;           // cells of a vertex row
+constexpr int kStripTries = 64;         // beginnings tried for its walk
+constexpr size_t kSmemSm = 227 * 1024;  // shared memory one SM gives to its CTAs
+constexpr size_t kSmemCta = 1024;       // the part the system takes of each CTA's share
+
+// marks of an edge row's record: the first and the last cell of a fan around
+// the edge; a closed fan ends at the vertex it began with
+constexpr uint32_t kFanBegin = 1u, kFanEnd = 2u, kFanClosed = 4u;
+
+// marks of a vertex row's record, beside the vertex it fetches: no cell yet
+// (the first two vertices of a strip); the next cell keeps the older one of
+// the last two vertices
+constexpr uint32_t kStripLoad = 0x80000000u, kStripKeep = 0x40000000u, kStripVertex = 0x3fffffffu;
+
+// kinds of rows
+enum { KIND_V = 0, KIND_E = 1, KIND_F = 2 };
+
+__host__ __device__ constexpr int dofs_of(int deg) { return deg == 1 ? 4 : (deg == 2 ? 10 : 20); }
+
+// kind of the node at local index i
+__device__ __forceinline__ int kind_of(int deg, int i) { return i < 4 ? KIND_V : (deg < 3 || i < 16 ? KIND_E : KIND_F); }
+
+// local edge {u, v} in the order (2,3),(1,3),(1,2),(0,3),(0,2),(0,1)
+__device__ __forceinline__ int edge_id(int u, int v) {
+  const int lo = min(u, v), hi = max(u, v);
+  return lo == 0 ? 6 - hi : (lo == 1 ? 4 - hi : 0);
+}
+// local dof of the P2 node of edge {x, y}; of the P3 node near x on it
+__device__ __forceinline__ int p2_edge(int x, int y) { return 4 + edge_id(x, y); }
+__device__ __forceinline__ int p3_edge(int x, int y) { return 4 + 2 * edge_id(x, y) + (x < y ? 0 : 1); }
+
+// ---------------------------------------------------------------------------
+// plan
+// ---------------------------------------------------------------------------
+struct PlanArgs {
+  int64_t num_cells, num_rows;
+  int k, deg;
+  const int32_t* geom;
+  const int32_t* dofs;
+  const uint8_t* pos;
+  const int32_t* row_ptr;  // first scalar row of block row R at R * bs
+  int bs;
+  int32_t* inc_ptr;
+  int32_t* inc;
+  unsigned* fail;
+};
+
+__global__ void k_rows_count(const PlanArgs a, int32_t* __restrict__ cnt, unsigned* __restrict__ kmask) {
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= a.num_cells) return;
+  const int32_t* d = a.dofs + c * a.k;
+  for (int i = 0; i < a.k; ++i) {
+    const int32_t r = d[i];
+    if (r < 0 || r >= a.num_rows) {
+      *a.fail = 1u;
+      return;
+    }
+    // a step adds to all its columns at once: they have to differ
+    for (int j = 0; j < i; ++j)
+      if (d[j] == r) *a.fail = 1u;
+    atomicAdd(cnt + r, 1);
+    const unsigned bit = 1u << kind_of(a.deg, i);
+    if (!(kmask[r] & bit)) atomicOr(kmask + r, bit);
+  }
+}
+
+__global__ void k_rows_fill(const PlanArgs a, int32_t* __restrict__ cursor) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= a.num_cells * a.k) return;
+  const int32_t r = a.dofs[t];
+  a.inc[atomicAdd(cursor + r, 1)] = (int32_t)t;
+}
+
+// sort key of a row: kind, window of 1024 rows (so that a warp's rows stay
+// close in memory), number of cells
+__global__ void k_rows_keys(const PlanArgs a, const int32_t* __restrict__ cnt, const unsigned* __restrict__ kmask,
+                            uint32_t* __restrict__ key, int32_t* __restrict__ row, int* __restrict__ kinds) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= a.num_rows) return;
+  const unsigned m = kmask[r];
+  if (m & (m - 1)) *a.fail = 1u;  // a node that is a vertex here and an edge node there
+  const int kind = m & 4u ? KIND_F : (m & 2u ? KIND_E : KIND_V);
+  const int n = min(cnt[r], 255);
+  key[r] = ((uint32_t)kind << 30) | ((uint32_t)(r >> 10) << 8) | (uint32_t)n;
+  row[r] = (int32_t)r;
+  atomicAdd(kinds + kind, 1);
+}
+
+// the cell's vertices in the row's order: positions p[0..3]
+__device__ __forceinline__ void row_order(int deg, int i, const int (&g)[4], int (&p)[4]) {
+  const int lo[6] = {2, 1, 1, 0, 0, 0}, hi[6] = {3, 3, 2, 3, 2, 1};
+  if (i < 4) {
+    p[0] = i;
+    int q = 1;
+    for (int v = 0; v < 4; ++v)
+      if (v != i) p[q++] = v;
+  } else if (deg == 2 || i < 16) {
+    const int e = deg == 2 ? i - 4 : (i - 4) / 2;
+    int u = lo[e], v = hi[e];
+    // P2: the lower mesh vertex first; P3: the vertex the node is near to
+    const bool swap = deg == 2 ? g[u] > g[v] : ((i - 4) & 1);
+    if (swap) {
+      const int t = u;
+      u = v;
+      v = t;
+    }
+    p[0] = u;
+    p[1] = v;
+    int q = 2;
+    for (int w = 0; w < 4; ++w)
+      if (w != u && w != v) p[q++] = w;
+  } else {
+    const int f = i - 16;
+    int q = 0;
+    for (int v = 0; v < 4; ++v)
+      if (v != f) p[q++] = v;
+    for (int s = 0; s < 2; ++s)  // the face's vertices by their mesh index
+      for (int t = 0; t < 2 - s; ++t)
+        if (g[p[t]] > g[p[t + 1]]) {
+          const int w = p[t];
+          p[t] = p[t + 1];
+          p[t + 1] = w;
+        }
+    p[3] = f;
+  }
+}
+
+// slots of the columns every cell of the row has, packed one byte each
+// (V: the row itself; E: a, b, the row, P3: the edge's other node)
+__device__ __forceinline__ uint32_t own_slots(int deg, int kind, const uint8_t* q, int i, const int (&p)[4]) {
+  if (kind == KIND_V) return q[i];
+  uint32_t w = q[p[0]] | ((uint32_t)q[p[1]] << 8) | ((uint32_t)q[i] << 16);
+  if (deg == 3) w |= (uint32_t)q[p3_edge(p[1], p[0])] << 24;
+  return w;
+}
+
+struct PartArgs {
+  int kind;
+  int64_t nrows, ngroups;
+  const int32_t* rows;   // [nrows] rows of this kind in walk order
+  int4* own;             // [ngroups*32]
+  int32_t* steps;        // [ngroups+1] records of the longest row of each group, then their prefix sum
+  uint4* rec;
+  uint2* rec1;           // P1 records
+  int32_t* cell;
+  unsigned* gaps;        // set when a row has slots that no cell adds to
+  int parts;             // vertex rows: warps that share a group's cells
+};
+
+__device__ __forceinline__ void load_cell(const PlanArgs& a, int32_t t, int64_t& c, int& i, int (&g)[4]) {
+  c = t / a.k;
+  i = t - (int32_t)c * a.k;
+  const int4 v = reinterpret_cast<const int4*>(a.geom)[c];
+  g[0] = v.x;
+  g[1] = v.y;
+  g[2] = v.z;
+  g[3] = v.w;
+}
+
+// The cells of a vertex row as strips of the triangles opposite the vertex,
+// cut into `parts` of nearly as many cells: emit(part, cell entry, its three
+// other vertices, flags) for each step, cell entry -1 for the two steps that
+// begin a strip; returns the steps of the longest part.  `code` says how the
+// first strip begins: its triangle, which of its vertices is left first, and
+// which way it goes at a tie.
+template <typename Emit>
+__device__ int walk_star(const PlanArgs& a, const int32_t* inc, int n, int parts, int code, Emit&& emit) {
+  int tv[kMaxStar][3];           // mesh vertices opposite the row's
+  uint32_t used[kMaxStar / 32];
+  for (int q = 0; q < kMaxStar / 32; ++q) used[q] = 0u;
+  for (int t = 0; t < n; ++t) {
+    int64_t c;
+    int i, g[4];
+    load_cell(a, inc[t], c, i, g);
+    int q = 0;
+    for (int v = 0; v < 4; ++v)
+      if (v != i) tv[t][q++] = g[v];
+  }
+  auto is_used = [&](int t) { return (used[t >> 5] >> (t & 31)) & 1u; };
+  auto has = [&](int t, int v) { return tv[t][0] == v || tv[t][1] == v || tv[t][2] == v; };
+  // the free triangle with vertices u and v, -1 if there is none
+  auto find = [&](int u, int v) {
+    for (int t = 0; t < n; ++t)
+      if (!is_used(t) && has(t, u) && has(t, v)) return t;
+    return -1;
+  };
+  auto third = [&](int t, int u, int v) {
+    for (int q = 0; q < 3; ++q)
+      if (tv[t][q] != u && tv[t][q] != v) return tv[t][q];
+    return u;
+  };
+  int steps = 0, longest = 0, left = n, first = 0, part = 0, done = 0;
+  auto next_part = [&]() {  // after `done` cells
+    if (part + 1 < parts && done >= (part + 1) * n / parts) {
+      ++part;
+      longest = max(longest, steps);
+      steps = 0;
+      return true;
+    }
+    return false;
+  };
+  bool begun = false;
+  while (left > 0) {
+    while (begun && is_used(first)) ++first;
+    int t = begun ? first : code / 6;
+    used[t >> 5] |= 1u << (t & 31);
+    --left;
+    // its vertices, so that the strip can go on over (q, r)
+    int p = tv[t][0], q = tv[t][1], r = tv[t][2];
+    if (!begun) {
+      const int turn = code / 2 % 3;
+      p = tv[t][turn];
+      q = tv[t][(turn + 1) % 3];
+      r = tv[t][(turn + 2) % 3];
+      begun = true;
+    } else if (find(q, r) < 0) {
+      if (find(p, r) >= 0) {
+        const int w = p;
+        p = q;
+        q = w;
+      } else if (find(p, q) >= 0) {
+        const int w = p;
+        p = r;
+        r = w;
+      }
+    }
+    emit(part, -1, p, 0, 0, kStripLoad);
+    emit(part, -1, q, 0, 0, kStripLoad);
+    steps += 2;
+    while (true) {
+      const int t1 = find(q, r), t2 = find(p, r);
+      int next = t1;
+      bool keep = false;
+      if (t2 >= 0) {
+        if (t1 < 0) {
+          keep = true;
+        } else {
+          // towards the triangle with fewer free neighbours
+          auto degree = [&](int x, int u, int v) {
+            const int w = third(x, u, v);
+            return (find(u, w) != x && find(u, w) >= 0 ? 1 : 0) + (find(v, w) != x && find(v, w) >= 0 ? 1 : 0);
+          };
+          keep = degree(t2, p, r) < degree(t1, q, r) + (code & 1);
+        }
+        if (keep) next = t2;
+      }
+      emit(part, t, r, p, q, keep ? kStripKeep : 0u);
+      ++steps;
+      ++done;
+      const bool cut = next_part();
+      if (next < 0) break;
+      if (!keep) p = q;
+      q = r;
+      r = third(next, p, q);
+      t = next;
+      if (cut) {
+        emit(part, -1, p, 0, 0, kStripLoad);
+        emit(part, -1, q, 0, 0, kStripLoad);
+        steps += 2;
+      }
+      used[t >> 5] |= 1u << (t & 31);
+      --left;
+    }
+  }
+  return max(longest, steps);
+}
+
+// per row: its cells in ascending order, its own vertices and slots; per
+// group the longest walk
+__global__ void k_rows_head(const PlanArgs a, const PartArgs p) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t g32 = t >> 5;
+  if (g32 >= p.ngroups) return;
+  int4 own = make_int4(-1, -1, -1, 0);
+  int n = 0;
+  if (t < p.nrows) {
+    const int32_t r = p.rows[t];
+    const int32_t lo = a.inc_ptr[r];
+    n = a.inc_ptr[r + 1] - lo;
+    int32_t* inc = a.inc + lo;
+    for (int q = 1; q < n; ++q) {
+      const int32_t v = inc[q];
+      int s = q;
+      for (; s > 0 && inc[s - 1] > v; --s) inc[s] = inc[s - 1];
+      inc[s] = v;
+    }
+    own.x = r;
+    for (int q = 0; q < n; ++q) {
+      int64_t c;
+      int i, g[4], o[4];
+      load_cell(a, inc[q], c, i, g);
+      row_order(a.deg, i, g, o);
+      const uint32_t w = own_slots(a.deg, p.kind, a.pos + (c * a.k + i) * a.k, i, o);
+      const int va = g[o[0]], vb = p.kind == KIND_V ? -1 : g[o[1]];
+      if (q == 0) {
+        own.y = va;
+        own.z = vb;
+        own.w = (int)w;
+      } else if (p.kind != KIND_F && (own.y != va || own.z != vb || (uint32_t)own.w != w)) {
+        *a.fail = 1u;  // one dof, several vertices or edges
+      }
+    }
+    if (p.kind == KIND_V) {
+      if (n > kMaxStar) *a.fail = 1u;
+      else if (n > 0) {
+        // the beginning whose walk has the fewest steps; one strip around the
+        // whole star, n + 2 steps, is found in two or three tries as a rule
+        auto steps_of = [&](int parts, int code) {
+          return walk_star(a, inc, n, parts, code, [](int, int, int, int, int, uint32_t) {});
+        };
+        int best = 0, least = steps_of(1, 0);
+        for (int code = 1; code < min(6 * n, kStripTries) && least > n + 2; ++code) {
+          const int steps = steps_of(1, code);
+          if (steps < least) {
+            least = steps;
+            best = code;
+          }
+        }
+        own.z = best;
+        n = p.parts == 1 ? least : steps_of(p.parts, best);
+      }
+    }
+  }
+  p.own[t] = own;
+  for (int o = 16; o > 0; o >>= 1) n = max(n, __shfl_xor_sync(kAll, n, o));
+  if ((t & 31) == 0) p.steps[g32] = n * p.parts;
+}
+
+// the records of every (step, lane)
+__global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t g32 = t >> 5;
+  const int lane = (int)(t & 31);
+  if (g32 >= p.ngroups) return;
+  int n = 0;
+  const int32_t* inc = nullptr;
+  int32_t r = -1;
+  if (t < p.nrows) {
+    r = p.rows[t];
+    inc = a.inc + a.inc_ptr[r];
+    n = a.inc_ptr[r + 1] - a.inc_ptr[r];
+  }
+  const int64_t s0 = p.steps[g32];
+  const int ns = p.steps[g32 + 1] - p.steps[g32];
+  uint64_t used = 0;  // edge rows: cells already listed (all of them below 64)
+  int last = -1;      // mesh vertex the next cell around the edge shares
+  int fan = -1;       // the vertex its fan began with
+  uint32_t seen[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};  // slots some cell adds to
+  uint32_t written[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  auto mark = [&](uint32_t b) { seen[b >> 5] |= 1u << (b & 31u); };
+  auto write = [&](uint32_t b) {
+    if ((written[b >> 5] >> (b & 31u)) & 1u) *a.fail = 1u;
+    written[b >> 5] |= 1u << (b & 31u);
+  };
+  if (p.kind == KIND_V) {
+    const int np = ns / p.parts;  // steps of a part
+    int at_part = -1, s = 0;
+    auto rest = [&]() {  // the part's steps without a cell
+      for (; at_part >= 0 && s < np; ++s) {
+        const int64_t at = (s0 + at_part * np + s) * 32 + lane;
+        p.cell[at] = 0;
+        if (a.deg == 1) p.rec1[at] = make_uint2(kStripLoad, 0u);
+        else p.rec[at] = make_uint4(kStripLoad, 0u, 0u, 0u);
+      }
+    };
+    if (n > 0 && n <= kMaxStar)
+      walk_star(a, inc, n, p.parts, p.own[t].z, [&](int part, int t, int r3, int p3, int q3, uint32_t flags) {
+        while (at_part < part) {
+          rest();
+          ++at_part;
+          s = 0;
+        }
+        const int64_t at = (s0 + part * np + s++) * 32 + lane;
+        uint4 w = make_uint4((uint32_t)r3 | flags, 0u, 0u, 0u);
+        p.cell[at] = 0;
+        if (t >= 0) {
+          int64_t c;
+          int i, g[4];
+          load_cell(a, inc[t], c, i, g);
+          int lp = 0, lq = 0, lr = 0;
+          for (int v = 0; v < 4; ++v) {
+            if (v == i) continue;
+            if (g[v] == p3) lp = v;
+            else if (g[v] == q3) lq = v;
+            else lr = v;
+          }
+          const uint8_t* q = a.pos + (c * a.k + i) * a.k;
+          auto B = [&](int j) -> uint32_t { return q[j]; };
+          for (int j = 0; j < a.k; ++j) mark(B(j));
+          p.cell[at] = (int32_t)c;
+          w.y = B(lp) | (B(lq) << 8) | (B(lr) << 16);
+          if (a.deg == 2) {
+            w.y |= B(p2_edge(i, lp)) << 24;
+            w.z = B(p2_edge(i, lq)) | (B(p2_edge(i, lr)) << 8) | (B(p2_edge(lp, lq)) << 16) |
+                  (B(p2_edge(lp, lr)) << 24);
+            w.w = B(p2_edge(lq, lr));
+          }
+        }
+        if (a.deg == 1) p.rec1[at] = make_uint2(w.x, w.y);
+        else p.rec[at] = w;
+      });
+    while (at_part < p.parts) {
+      rest();
+      ++at_part;
+      s = 0;
+    }
+  }
+  for (int s = 0; s < (p.kind == KIND_E ? ns : 0); ++s) {
+    const int64_t at = (s0 + s) * 32 + lane;
+    if (s >= n) {
+      p.cell[at] = 0;
+      p.rec[at] = make_uint4(kAll, kAll, 0u, 0u);
+      continue;
+    }
+    int64_t c;
+    int i, g[4], o[4];
+    uint32_t flags = kFanBegin | kFanEnd;  // edge rows: a fan of one cell
+    if (n <= 64) {
+      // the next unlisted cell with the last vertex; else one that has a
+      // vertex no other unlisted cell has (an end of an open fan); else the first
+      int pick = -1, end = -1, first = -1;
+      for (int q = 0; q < n && pick < 0; ++q) {
+        if ((used >> q) & 1u) continue;
+        load_cell(a, inc[q], c, i, g);
+        row_order(a.deg, i, g, o);
+        if (first < 0) first = q;
+        if (last >= 0) {
+          if (g[o[2]] == last || g[o[3]] == last) pick = q;
+          continue;
+        }
+        int shared[2] = {0, 0};
+        for (int q2 = 0; q2 < n; ++q2) {
+          if (q2 == q || ((used >> q2) & 1u)) continue;
+          int64_t c2;
+          int i2, g2[4], o2[4];
+          load_cell(a, inc[q2], c2, i2, g2);
+          row_order(a.deg, i2, g2, o2);
+          for (int e = 0; e < 2; ++e) shared[e] |= g[o[2 + e]] == g2[o2[2]] || g[o[2 + e]] == g2[o2[3]];
+        }
+        if (end < 0 && !(shared[0] && shared[1])) {
+          end = q;
+          last = -1;
+        }
+      }
+      if (pick < 0) pick = end >= 0 ? end : first;
+      used |= uint64_t(1) << pick;
+      load_cell(a, inc[pick], c, i, g);
+      row_order(a.deg, i, g, o);
+      bool swap = last >= 0 && g[o[3]] == last;
+      if (last < 0 || (g[o[2]] != last && g[o[3]] != last)) {
+        // a new fan: begin with the vertex that no other unlisted cell has
+        bool s2 = false, s3 = false;
+        for (int q2 = 0; q2 < n; ++q2) {
+          if ((used >> q2) & 1u) continue;
+          int64_t c2;
+          int i2, g2[4], o2[4];
+          load_cell(a, inc[q2], c2, i2, g2);
+          row_order(a.deg, i2, g2, o2);
+          s2 |= g[o[2]] == g2[o2[2]] || g[o[2]] == g2[o2[3]];
+          s3 |= g[o[3]] == g2[o2[2]] || g[o[3]] == g2[o2[3]];
+        }
+        swap = s2 && !s3;
+      }
+      if (swap) {
+        const int w = o[2];
+        o[2] = o[3];
+        o[3] = w;
+      }
+      flags = 0u;
+      if (last < 0 || g[o[2]] != last) {
+        flags |= kFanBegin;
+        fan = g[o[2]];
+      }
+      last = g[o[3]];
+      // the fan ends when no unlisted cell has its last vertex
+      bool more = false;
+      for (int q2 = 0; q2 < n && !more; ++q2) {
+        if ((used >> q2) & 1u) continue;
+        int64_t c2;
+        int i2, g2[4], o2[4];
+        load_cell(a, inc[q2], c2, i2, g2);
+        row_order(a.deg, i2, g2, o2);
+        more = g2[o2[2]] == last || g2[o2[3]] == last;
+      }
+      if (!more) {
+        flags |= kFanEnd;
+        if (last == fan) flags |= kFanClosed;
+        last = -1;
+      }
+    } else {
+      load_cell(a, inc[s], c, i, g);
+      row_order(a.deg, i, g, o);
+    }
+    const uint8_t* q = a.pos + (c * a.k + i) * a.k;
+    auto B = [&](int j) -> uint32_t { return q[j]; };
+    for (int j = 0; j < a.k; ++j) mark(B(j));
+    p.cell[at] = (int32_t)c;
+    {
+      uint4 w;
+      w.x = (uint32_t)g[o[2]];
+      w.y = (uint32_t)g[o[3]];
+      w.z = B(o[2]) | (B(o[3]) << 8) | (B(p2_edge(o[0], o[2])) << 16) | (B(p2_edge(o[0], o[3])) << 24);
+      w.w = B(p2_edge(o[1], o[2])) | (B(p2_edge(o[1], o[3])) << 8) | (B(p2_edge(o[2], o[3])) << 16) |
+            (flags << 24);
+      p.rec[at] = w;
+      // the walk writes a slot once (twice at the end of a closed fan): cells
+      // that overlap, or three at one face, are left to the scatter
+      write(w.z & 0xffu);
+      write((w.z >> 16) & 0xffu);
+      write(w.w & 0xffu);
+      write((w.w >> 16) & 0xffu);
+      if ((flags & kFanEnd) && !(flags & kFanClosed)) {
+        write((w.z >> 8) & 0xffu);
+        write(w.z >> 24);
+        write((w.w >> 8) & 0xffu);
+      }
+    }
+  }
+  if (r >= 0) {
+    int covered = 0;
+    for (int q = 0; q < 8; ++q) covered += __popc(seen[q]);
+    if (covered != a.row_ptr[r + 1] - a.row_ptr[r]) *p.gaps = 1u;
+  }
+}
+
+__global__ void k_rows_pad_x(const double* __restrict__ x, int64_t n, double4* __restrict__ x4) {
+  const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (v < n) x4[v] = make_double4(x[3 * v], x[3 * v + 1], x[3 * v + 2], 0.0);
+}
+
+__global__ void k_rows_same_map(const int32_t* __restrict__ m, const int32_t* __restrict__ g, int64_t n,
+                                unsigned* __restrict__ differ) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t < n && m[t] != g[t]) *differ = 1u;
+}
+
+// bit s of the mask: the column of slot s is a BC column
+__global__ void k_rows_bc_mask(const int32_t* __restrict__ col, int64_t nnz, const uint8_t* __restrict__ markers,
+                               uint32_t* __restrict__ mask) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const unsigned b = __ballot_sync(kAll, q < nnz && markers[col[q]] != 0);
+  if ((threadIdx.x & 31) == 0 && q < nnz) mask[q >> 5] = b;
+}
+// bit 0: a BC row; bit 1: a row with a BC column
+__global__ void k_rows_bc_flags(const int32_t* __restrict__ row_ptr, int64_t num_rows,
+                                const uint8_t* __restrict__ markers, const uint32_t* __restrict__ mask,
+                                uint8_t* __restrict__ flags) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= num_rows) return;
+  const int32_t lo = row_ptr[r], hi = row_ptr[r + 1];
+  uint32_t any = 0u;
+  for (int32_t w = lo >> 5; w <= (hi - 1) >> 5 && lo < hi; ++w) {
+    uint32_t m = mask[w];
+    if (w == lo >> 5) m &= kAll << (lo & 31);
+    if (w == (hi - 1) >> 5) m &= kAll >> (31 - ((hi - 1) & 31));
+    any |= m;
+  }
+  flags[r] = (uint8_t)((markers[r] ? 1 : 0) | (any ? 2 : 0));
+}
+
+// ---------------------------------------------------------------------------
+// assembly
+// ---------------------------------------------------------------------------
+struct WalkArgs {
+  int64_t ngroups;
+  const int4* __restrict__ own;
+  const int32_t* __restrict__ steps;
+  const uint4* __restrict__ rec;
+  const uint2* __restrict__ rec1;
+  const int32_t* __restrict__ cell;
+  const double4* __restrict__ x4;
+  int stride;     // doubles between the segments of a warp's rows (odd)
+  int gaps;       // some rows have slots that no cell adds to
+  const double* __restrict__ coef;   // DG0: [cells]; P1: [vertices]
+  double coef_const;
+  const int32_t* __restrict__ row_ptr;
+  const uint8_t* __restrict__ flags;  // BC flags of the rows, or null
+  const uint32_t* __restrict__ mask;  // bit s: the column of slot s is a BC column
+  double diagonal;   // stored on BC rows (with zero)
+  int zero;
+  double* __restrict__ values;
+};
+
+struct V3 {
+  double x, y, z;
+};
+__device__ __forceinline__ V3 operator-(const V3& a, const V3& b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ double dot(const V3& a, const V3& b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
+__device__ __forceinline__ V3 cross(const V3& a, const V3& b) {
+  return {fma(a.y, b.z, -(a.z * b.y)), fma(a.z, b.x, -(a.x * b.z)), fma(a.x, b.y, -(a.y * b.x))};
+}
+__device__ __forceinline__ V3 neg_sum(const V3& a, const V3& b, const V3& c) {
+  return {-(a.x + b.x + c.x), -(a.y + b.y + c.y), -(a.z + b.z + c.z)};
+}
+__device__ __forceinline__ V3 load_x(const double4* __restrict__ x4, int v) {
+  const double2* p = reinterpret_cast<const double2*>(x4 + v);
+  const double2 a = __ldg(p);
+  const double b = __ldg(reinterpret_cast<const double*>(p + 1));
+  return {a.x, a.y, b};
+}
+
+// a lane's row in the value array, fetched before the walk
+struct RowAt {
+  int lo = 0, len = 0, fl = 0;
+};
+__device__ __forceinline__ RowAt row_at(const WalkArgs& a, int row) {
+  RowAt r;
+  if (row >= 0) {
+    r.lo = __ldg(a.row_ptr + row);
+    r.len = __ldg(a.row_ptr + row + 1) - r.lo;
+    if (a.flags) r.fl = __ldg(a.flags + row);
+  }
+  return r;
+}
+
+// The warp's 32 row segments (lane l's at acc + l * stride) to their rows.
+// First the segments of rows that a BC touches take their zeros (and a BC row
+// `diagonal` at its own slot), then all rows are stored, or added with zero == 0.
+// A warp takes the `count` rows from `first` on.
+__device__ __forceinline__ void store_rows(const WalkArgs& a, double* acc, const RowAt& at, int own_slot, int lane,
+                                           int first, int count) {
+  const unsigned mine = count == 32 ? kAll : ((1u << count) - 1u) << first;
+  __syncwarp();
+  // about every second warp has such rows, a few of them: four at a time, so
+  // that their mask words are fetched together
+  for (unsigned todo = __ballot_sync(kAll, at.fl != 0) & mine; todo;) {
+    int rr[4], rlo[4], rlen[4], rfl[4], rown[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      rr[q] = todo ? __ffs(todo) - 1 : 0;
+      rlo[q] = __shfl_sync(kAll, at.lo, rr[q]);
+      const int len = __shfl_sync(kAll, at.len, rr[q]);
+      rlen[q] = todo ? len : 0;
+      rfl[q] = __shfl_sync(kAll, at.fl, rr[q]);
+      rown[q] = __shfl_sync(kAll, own_slot, rr[q]);
+      todo &= todo - 1;
+    }
+    const int most = max(max(rlen[0], rlen[1]), max(rlen[2], rlen[3]));
+    for (int s = lane; s < most; s += 32) {
+      uint32_t m[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int w = rlo[q] + s;
+        m[q] = s < rlen[q] ? ((rfl[q] & 1) ? 1u : (__ldg(a.mask + (w >> 5)) >> (w & 31)) & 1u) : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (m[q]) acc[rr[q] * a.stride + s] = (rfl[q] & 1) && s == rown[q] ? a.diagonal : 0.0;
+    }
+  }
+  __syncwarp();
+  const int len0 = __shfl_sync(kAll, at.len, 0);
+  if (a.zero && len0 > 0 && __all_sync(kAll, at.len == len0)) {
+    // 32 rows of one length: the lanes go through their entries without a gap
+    const int jump = 32 / len0, rest = 32 - jump * len0, end = first + count;
+    int rr = lane / len0, s = lane - rr * len0;
+    rr += first;
+#pragma unroll 4
+    for (int it = 0; it < count * len0; it += 32) {
+      const int rlo = __shfl_sync(kAll, at.lo, rr);
+      if (rr < end) a.values[rlo + s] = acc[rr * a.stride + s];
+      rr += jump;
+      s += rest;
+      if (s >= len0) {
+        s -= len0;
+        ++rr;
+      }
+    }
+    return;
+  }
+#pragma unroll 4
+  for (int rr = first; rr < first + count; ++rr) {
+    const int rlo = __shfl_sync(kAll, at.lo, rr), rlen = __shfl_sync(kAll, at.len, rr);
+    const double* seg = acc + rr * a.stride;
+    for (int s = lane; s < rlen; s += 32) {
+      const double v = seg[s];
+      if (a.zero) a.values[rlo + s] = v;
+      else a.values[rlo + s] += v;
+    }
+  }
+}
+
+// One warp a CTA: a finished warp's shared memory goes to the next one at once
+// (P2 n=96: 1.15 ms against 1.22 ms with CTAs of two and four warps).
+// CTAs per SM to fit in registers (fewer registers spill, more leave too few
+// warps):
+constexpr int kMinV1 = 20, kMinV2 = 13, kMinE = 20;
+
+// The kernels of one call write different rows: the later one starts while
+// the earlier one runs (programmatic dependent launch) and ends after it, so
+// that what follows in the stream waits for both.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void end_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+
+// Vertex rows (P1: all rows): the cells around vertex a as strips, each with
+// its three other vertices p, q, r, where r is fetched and p, q are two of
+// the cell's before.
+// PARTS warps share the rows of a group, each with its part of every row's
+// cells and segments of its own, which are added up at the end.
+template <int DEG, int COEF, int PARTS>
+__global__ void __launch_bounds__(32 * PARTS, (DEG == 1 ? kMinV1 : kMinV2) / PARTS) k_rows_v(const WalkArgs a) {
+  let_next_start();
+  extern __shared__ double smem[];
+  const int lane = threadIdx.x & 31, part = PARTS == 1 ? 0 : threadIdx.x >> 5;
+  const int64_t g = blockIdx.x;
+  double* acc = smem + part * (32 * a.stride);
+  double* seg = acc + lane * a.stride;
+  const int4 own = __ldg(a.own + g * 32 + lane);
+  int s0 = __ldg(a.steps + g);
+  const int ns = (__ldg(a.steps + g + 1) - s0) / PARTS;
+  s0 += part * ns;
+  const uint4* rec = a.rec + (int64_t)s0 * 32 + lane;
+  const uint2* rec1 = a.rec1 + (int64_t)s0 * 32 + lane;
+  const int32_t* cell = a.cell + (int64_t)s0 * 32 + lane;
+  int c1 = 0, c2 = 0;  // the records' cells (DG0)
+  auto record = [&](int s) {
+    uint4 w = make_uint4(kStripLoad, 0u, 0u, 0u);
+    c1 = c2;
+    if (s < ns) {
+      if constexpr (COEF == FE_COEFF_DG0) c2 = __ldg(cell + s * 32);
+      if constexpr (DEG == 1) {
+        const uint2 h = __ldg(rec1 + s * 32);
+        w.x = h.x;
+        w.y = h.y;
+      } else {
+        w = __ldg(rec + s * 32);
+      }
+    }
+    return w;
+  };
+  // the records run two steps ahead, the coordinates and the coefficient one
+  uint4 w1 = record(0), w2 = record(1);
+  const RowAt at = row_at(a, own.x);
+  V3 xa{0.0, 0.0, 0.0}, xr, ep{0.0, 0.0, 0.0}, eq{0.0, 0.0, 0.0};
+  double ka = 1.0, kp = 1.0, kq = 1.0, kn = a.coef_const;
+  auto fetch = [&](const uint4& w) {
+    const int v = (int)(w.x & kStripVertex);
+    xr = load_x(a.x4, v);
+    if constexpr (COEF == FE_COEFF_P1) kn = __ldg(a.coef + v);
+    if constexpr (COEF == FE_COEFF_DG0) kn = __ldg(a.coef + c1);
+  };
+  fetch(w1);
+  if (own.y >= 0) {
+    xa = load_x(a.x4, own.y);
+    if constexpr (COEF == FE_COEFF_P1) ka = __ldg(a.coef + own.y);
+  }
+  for (int s = 0; s < a.stride; ++s) seg[s] = 0.0;
+  double diag = 0.0;
+  for (int s = 0; s < ns; ++s) {
+    const uint4 w = w1;
+    w1 = w2;
+    w2 = record(s + 2);
+    const V3 er = xr - xa;
+    const double kr = kn;
+    fetch(w1);
+    if (!(w.x & kStripLoad)) {
+      const V3 gp = cross(eq, er), gq = cross(er, ep), gr = cross(ep, eq);
+      const V3 ga = neg_sum(gp, gq, gr);
+      const double rdet = 1.0 / fabs(dot(ep, gp));
+      const double ap = dot(ga, gp), aq = dot(ga, gq), ar = dot(ga, gr);
+      const double aa = -(ap + aq + ar);
+      constexpr int NV = DEG == 1 ? 3 : 9;
+      double v[NV];  // columns p, q, r, ap, aq, ar, pq, pr, qr
+      if constexpr (DEG == 1) {
+        // k |T| grad.grad with the cell mean of k (exact: the gradients are constant)
+        double f;
+        if constexpr (COEF == FE_COEFF_P1) f = (1.0 / 24.0) * ((ka + kp) + (kq + kr)) * rdet;
+        else f = (1.0 / 6.0) * kr * rdet;
+        v[0] = f * ap;
+        v[1] = f * aq;
+        v[2] = f * ar;
+        diag = fma(f, aa, diag);
+      } else if constexpr (COEF == FE_COEFF_P1) {
+        const double S = (ka + kp) + (kq + kr);
+        const double f = (1.0 / 720.0) * rdet, f4 = 4.0 * f, m2 = -2.0 * S;
+        diag = fma(f * fma(14.0, S, 16.0 * ka), aa, diag);
+        v[0] = f * fma(-8.0, ka + kp, m2) * ap;
+        v[1] = f * fma(-8.0, ka + kq, m2) * aq;
+        v[2] = f * fma(-8.0, ka + kr, m2) * ar;
+        // column ap: (2S + 10 k_a) ap + (-2S + 4 k_a - 2 k_p) aa
+        const double y = fma(10.0, ka, -m2), t = fma(4.0, ka, m2);
+        const double tp = fma(-2.0, kp, t), tq = fma(-2.0, kq, t), tr = fma(-2.0, kr, t);
+        v[3] = f4 * fma(y, ap, tp * aa);
+        v[4] = f4 * fma(y, aq, tq * aa);
+        v[5] = f4 * fma(y, ar, tr * aa);
+        // column pq: (-2S + 4 k_a - 2 k_p) aq + (-2S + 4 k_a - 2 k_q) ap
+        v[6] = f4 * fma(tp, aq, tq * ap);
+        v[7] = f4 * fma(tp, ar, tr * ap);
+        v[8] = f4 * fma(tq, ar, tr * aq);
+      } else {
+        const double f = (1.0 / 30.0) * kr * rdet;  // 4 k / 120
+        diag = fma(3.0 * f, aa, diag);
+        v[0] = -f * ap;
+        v[1] = -f * aq;
+        v[2] = -f * ar;
+        v[3] = f * fma(3.0, ap, -aa);
+        v[4] = f * fma(3.0, aq, -aa);
+        v[5] = f * fma(3.0, ar, -aa);
+        v[6] = -f * (ap + aq);
+        v[7] = -f * (ap + ar);
+        v[8] = -f * (aq + ar);
+      }
+      const uint32_t sl[9] = {w.y & 0xffu, (w.y >> 8) & 0xffu, (w.y >> 16) & 0xffu, w.y >> 24, w.z & 0xffu,
+                              (w.z >> 8) & 0xffu, (w.z >> 16) & 0xffu, w.z >> 24, w.w};
+      // a cell's columns differ: all reads before the writes
+      double o[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) o[q] = seg[sl[q]];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) seg[sl[q]] = o[q] + v[q];
+    }
+    if (!(w.x & kStripKeep)) {
+      ep = eq;
+      kp = kq;
+    }
+    eq = er;
+    kq = kr;
+  }
+  if (own.y >= 0) seg[own.w & 0xff] += diag;
+  if constexpr (PARTS > 1) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < 32 * a.stride; t += 32 * PARTS) {
+      double v = smem[t];
+#pragma unroll
+      for (int q = 1; q < PARTS; ++q) v += smem[q * (32 * a.stride) + t];
+      smem[t] = v;
+    }
+    __syncthreads();
+  }
+  constexpr int kRows = 32 / PARTS;
+  store_rows(a, smem, at, own.w & 0xff, lane, part * kRows, kRows);
+}
+
+// Edge rows of P2: node ab; the cells around the edge in fans, each with its
+// two other vertices c, d, where d is the next cell's c.  The columns c, ac
+// and bc take entries of the two cells with the face abc, one after the
+// other: their sum runs in registers and is written once, cd belongs to one
+// cell, and a, b and ab stay in registers, so the segment is written without
+// being read (but for the end of a closed fan).
+template <int COEF>
+__global__ void __launch_bounds__(32, kMinE) k_rows_e2(const WalkArgs a) {
+  extern __shared__ double smem[];
+  const int lane = threadIdx.x;
+  const int64_t g = blockIdx.x;
+  double* acc = smem;
+  double* seg = acc + lane * a.stride;
+  const int4 own = __ldg(a.own + g * 32 + lane);
+  const int s0 = __ldg(a.steps + g), ns = __ldg(a.steps + g + 1) - s0;
+  const uint4 none = make_uint4(kAll, kAll, 0u, 0u);
+  const uint4* rec = a.rec + (int64_t)s0 * 32 + lane;
+  const int32_t* cell = a.cell + (int64_t)s0 * 32 + lane;
+  // the records run two cells ahead, the coordinates and the coefficient one
+  uint4 wp = ns > 0 ? __ldg(rec) : none, wq = ns > 1 ? __ldg(rec + 32) : none;
+  const RowAt at = row_at(a, own.x);
+  V3 xa{0.0, 0.0, 0.0}, e1{0.0, 0.0, 0.0}, xd{0.0, 0.0, 0.0};
+  double ka = 1.0, kb = 1.0, kn = a.coef_const;
+  int c1 = 0, c2 = 0;  // the records' cells (DG0)
+  if constexpr (COEF == FE_COEFF_DG0) {
+    if (ns > 0) c1 = __ldg(cell);
+    if (ns > 1) c2 = __ldg(cell + 32);
+  }
+  auto fetch = [&](const uint4& w) {
+    if (w.y == kAll) return;
+    xd = load_x(a.x4, (int)w.y);
+    if constexpr (COEF == FE_COEFF_P1) kn = __ldg(a.coef + w.y);
+    if constexpr (COEF == FE_COEFF_DG0) kn = __ldg(a.coef + c1);
+  };
+  if (own.y >= 0) {
+    xa = load_x(a.x4, own.y);
+    e1 = load_x(a.x4, own.z) - xa;
+    if constexpr (COEF == FE_COEFF_P1) {
+      ka = __ldg(a.coef + own.y);
+      kb = __ldg(a.coef + own.z);
+    }
+  }
+  fetch(wp);
+  if (a.gaps)
+    for (int s = 0; s < a.stride; ++s) seg[s] = 0.0;
+  double va = 0.0, vb = 0.0, vab = 0.0;  // columns a, b and ab
+  double rc = 0.0, rac = 0.0, rbc = 0.0; // columns c, ac and bc so far
+  // one cell: c, its edge vector from a, e1 x c and its coefficient come from
+  // the cell before (or are fetched where a fan begins), d's go to the next
+  auto step = [&](const uint4& w, const uint4& wnext, V3& ec, V3& hc, double& kc, V3& ed, V3& hd, double& kd) {
+    if (w.y != kAll) {
+      if ((w.w >> 24) & kFanBegin) {
+        ec = load_x(a.x4, (int)w.x) - xa;
+        if constexpr (COEF == FE_COEFF_P1) kc = __ldg(a.coef + w.x);
+        rc = rac = rbc = 0.0;
+      }
+      ed = xd - xa;
+      const double k = kn;
+      kd = kn;
+      fetch(wnext);
+      hd = cross(e1, ed);
+      hc = cross(e1, ec);
+      // times det: grad b = c x d, grad c = -(e1 x d), grad d = e1 x c
+      const V3 gb = cross(ec, ed);
+      const V3 ga{hd.x - hc.x - gb.x, hd.y - hc.y - gb.y, hd.z - hc.z - gb.z};
+      const double rdet = 1.0 / fabs(dot(e1, gb));
+      const double ab = dot(ga, gb), ac = -dot(ga, hd), ad = dot(ga, hc), bc = -dot(gb, hd), bd = dot(gb, hc);
+      const double aa = -(ab + ac + ad), bb = -(ab + bc + bd);
+      double vd, vad, vbd, vcd;
+      if constexpr (COEF == FE_COEFF_P1) {
+        // integrals of k lambda_x lambda_y, in units of |det| / 720: S + k_x + k_y,
+        // twice that for x = y
+        const double S = (ka + kb) + (kc + kd);
+        const double f4 = (4.0 / 720.0) * rdet, f16 = (16.0 / 720.0) * rdet, m2 = -2.0 * S;
+        const double Sa = S + ka, Sb = S + kb;
+        const double Maa = fma(4.0, ka, -m2), Mbb = fma(4.0, kb, -m2), Mab = Sa + kb;
+        const double Mac = Sa + kc, Mad = Sa + kd, Mbc = Sb + kc, Mbd = Sb + kd;
+        vab = fma(f16, fma(Maa, bb, fma(Mbb, aa, 2.0 * Mab * ab)), vab);
+        va = fma(f4, fma(fma(10.0, ka, -m2), ab, fma(4.0, ka, fma(-2.0, kb, m2)) * aa), va);
+        vb = fma(f4, fma(fma(10.0, kb, -m2), ab, fma(4.0, kb, fma(-2.0, ka, m2)) * bb), vb);
+        const double ta = fma(-2.0, ka, m2), tb = fma(-2.0, kb, m2);
+        rc = fma(f4, fma(fma(4.0, kc, ta), bc, fma(4.0, kc, tb) * ac), rc);
+        vd = f4 * fma(fma(4.0, kd, ta), bd, fma(4.0, kd, tb) * ad);
+        rac = fma(f16, fma(Maa, bc, fma(Mac, ab, fma(Mab, ac, Mbc * aa))), rac);
+        vad = f16 * fma(Maa, bd, fma(Mad, ab, fma(Mab, ad, Mbd * aa)));
+        rbc = fma(f16, fma(Mbb, ac, fma(Mbc, ab, fma(Mab, bc, Mac * bb))), rbc);
+        vbd = f16 * fma(Mbb, ad, fma(Mbd, ab, fma(Mab, bd, Mad * bb)));
+        vcd = f16 * fma(Mac, bd, fma(Mad, bc, fma(Mbc, ad, Mbd * ac)));
+      } else {
+        const double f = (1.0 / 30.0) * k * rdet, f16 = 4.0 * f;  // 4 k / 120, 16 k / 120
+        vab = fma(2.0 * f16, (aa + bb) + ab, vab);
+        va = fma(f, fma(3.0, ab, -aa), va);
+        vb = fma(f, fma(3.0, ab, -bb), vb);
+        rc = fma(-f, ac + bc, rc);
+        vd = -f * (ad + bd);
+        rac = fma(f16, fma(2.0, bc, -ad), rac);
+        vad = f16 * fma(2.0, bd, -ac);
+        rbc = fma(f16, fma(2.0, ac, -bd), rbc);
+        vbd = f16 * fma(2.0, ad, -bc);
+        vcd = f16 * ((ac + ad) + (bc + bd));
+      }
+      seg[w.z & 0xffu] = rc;
+      seg[(w.z >> 16) & 0xffu] = rac;
+      seg[w.w & 0xffu] = rbc;
+      seg[(w.w >> 16) & 0xffu] = vcd;
+      rc = vd;
+      rac = vad;
+      rbc = vbd;
+      if ((w.w >> 24) & kFanEnd) {
+        double* pd = seg + ((w.z >> 8) & 0xffu);
+        double* pad = seg + (w.z >> 24);
+        double* pbd = seg + ((w.w >> 8) & 0xffu);
+        if ((w.w >> 24) & kFanClosed) {
+          rc += *pd;
+          rac += *pad;
+          rbc += *pbd;
+        }
+        *pd = rc;
+        *pad = rac;
+        *pbd = rbc;
+      }
+    }
+  };
+  V3 ep{0.0, 0.0, 0.0}, eq{0.0, 0.0, 0.0}, hp{0.0, 0.0, 0.0}, hq{0.0, 0.0, 0.0};
+  double kp = 1.0, kq = 1.0;
+  for (int s = 0; s < ns; ++s) {
+    uint4 w = wp;
+    wp = wq;
+    wq = s + 2 < ns ? __ldg(rec + (s + 2) * 32) : none;
+    if constexpr (COEF == FE_COEFF_DG0) {
+      c1 = c2;
+      if (s + 2 < ns) c2 = __ldg(cell + (s + 2) * 32);
+    }
+    step(w, wp, ep, hp, kp, eq, hq, kq);
+    ep = eq;
+    hp = hq;
+    kp = kq;
+  }
+  if (own.y >= 0) {
+    seg[own.w & 0xff] = va;
+    seg[(own.w >> 8) & 0xff] = vb;
+    seg[(own.w >> 16) & 0xff] = vab;
+  }
+  store_rows(a, acc, at, (own.w >> 16) & 0xff, lane, 0, 32);
+  end_after_previous();
+}
+
+unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
+
+int odd_at_least(int n) { return n | 1; }
+
+size_t segment_bytes(int stride) { return sizeof(double) * 32 * (size_t)stride; }
+
+template <typename K>
+void raise_smem(K kernel) {
+  FE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSm));
+}
+
+int degree_of(int kind) {
+  switch (kind) {
+    case FE_FORM_P1_STIFFNESS: return 1;
+    case FE_FORM_P2_STIFFNESS: return 2;
+    default: return 0;
+  }
+}
+
+void exclusive_scan(int32_t* v, int64_t n, cudaStream_t s) {
+  size_t tb = 0;
+  FE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, v, v, (int)n, s));
+  DevBuf<unsigned char> tmp(std::max<size_t>(1, tb));
+  FE_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, v, v, (int)n, s));
+  FE_CUDA(cudaStreamSynchronize(s));
+}
+
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  FE_CUDA(cudaStreamIsCapturing(s, &st));
+  return st != cudaStreamCaptureStatusNone;
+}
+
+// a P1 coefficient's dofmap is the mesh's own vertex numbering (then its
+// values can be fetched by mesh vertex); asked once per dofmap
+bool vertex_numbered(fe_form_s& f, const fe_dofmap_s& map, cudaStream_t s) {
+  fe_form_s::RowsPlan& P = *f.rows_plan;
+  if (P.map_id == map.id) return P.map_same;
+  if (capturing(s)) return false;
+  bool same = map.num_cells == f.mesh->num_cells && map.k == 4 && map.num_blocks >= f.mesh->num_nodes;
+  if (same && map.num_cells > 0) {
+    DevBuf<unsigned> differ(1);
+    FE_CUDA(cudaMemsetAsync(differ.p, 0, sizeof(unsigned), s));
+    const int64_t n = map.num_cells * 4;
+    k_rows_same_map<<<blocks_for(n, 256), 256, 0, s>>>(map.dofs.p, f.mesh->geom.p, n, differ.p);
+    FE_CUDA(cudaGetLastError());
+    unsigned h = 0;
+    FE_CUDA(cudaMemcpyAsync(&h, differ.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FE_CUDA(cudaStreamSynchronize(s));
+    same = h == 0;
+  }
+  P.map_id = map.id;
+  P.map_same = same;
+  return same;
+}
+
+void build_part(const PlanArgs& a, PartArgs p, fe_form_s::RowsPlan::Part& part, const int32_t* rows, cudaStream_t s) {
+  part.ngroups = p.ngroups;
+  part.parts = p.parts;
+  part.own.alloc((size_t)p.ngroups * 32);
+  part.steps.alloc((size_t)p.ngroups + 1);
+  DevBuf<unsigned> gaps(1);
+  FE_CUDA(cudaMemsetAsync(gaps.p, 0, sizeof(unsigned), s));
+  FE_CUDA(cudaMemsetAsync(part.steps.p, 0, part.steps.bytes(), s));
+  p.rows = rows;
+  p.own = part.own.p;
+  p.steps = part.steps.p;
+  p.gaps = gaps.p;
+  k_rows_head<<<blocks_for(p.ngroups * 32, 128), 128, 0, s>>>(a, p);
+  FE_CUDA(cudaGetLastError());
+  exclusive_scan(part.steps.p, p.ngroups + 1, s);
+  int32_t total = 0;
+  FE_CUDA(cudaMemcpyAsync(&total, part.steps.p + p.ngroups, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  unsigned bad = 0;
+  FE_CUDA(cudaMemcpyAsync(&bad, a.fail, sizeof(bad), cudaMemcpyDeviceToHost, s));
+  FE_CUDA(cudaStreamSynchronize(s));
+  if (bad) return;
+  const size_t nrec = (size_t)total * 32;
+  if (a.deg == 1) part.rec1.alloc(std::max<size_t>(1, nrec));
+  else part.rec.alloc(std::max<size_t>(1, nrec));
+  part.cell.alloc(std::max<size_t>(1, nrec));
+  p.rec = part.rec.p;
+  p.rec1 = part.rec1.p;
+  p.cell = part.cell.p;
+  k_rows_records<<<blocks_for(p.ngroups * 32, 128), 128, 0, s>>>(a, p);
+  FE_CUDA(cudaGetLastError());
+  unsigned g = 0;
+  FE_CUDA(cudaMemcpyAsync(&g, gaps.p, sizeof(g), cudaMemcpyDeviceToHost, s));
+  FE_CUDA(cudaStreamSynchronize(s));
+  part.gaps = g != 0;
+}
+
+template <int DEG, int COEF>
+void raise_v() {
+  raise_smem(k_rows_v<DEG, COEF, 1>);
+  raise_smem(k_rows_v<DEG, COEF, 2>);
+  raise_smem(k_rows_v<DEG, COEF, 4>);
+}
+template <int DEG>
+void raise_all() {
+  raise_v<DEG, FE_COEFF_CONSTANT>();
+  raise_v<DEG, FE_COEFF_DG0>();
+  raise_v<DEG, FE_COEFF_P1>();
+}
+
+}  // namespace
+
+void reset_rows_plan(fe_form_s& f) { f.rows_plan.reset(); }
+
+// Small meshes keep the scatter: a call's time is its launches there and the
+// plan would not pay.  On B200, us per call, walk / best scatter: P1 n=20
+// (48,000 cells) 8.4 / 9.1, n=32 (196,608) 13.7 / 16.7, n=45 28 / 35; P2 n=16
+// (24,576) 16 / 18, n=20 25 / 25, n=28 (131,712) 42 / 64.
+bool rows_default(const fe_form_s& f) {
+  const int64_t cells = f.mesh ? f.mesh->num_cells : 0;
+  switch (degree_of(f.kind)) {
+    case 1: return cells >= 98304;
+    case 2: return cells >= 65536;
+    default: return false;
+  }
+}
+
+// Builds the plan of a form bound to a plain pattern; leaves the form without
+// one where the walk does not apply (the assembly then takes the scatter):
+// kinds without a row walk, two different spaces, dofs that stand for several
+// mesh vertices or edges (periodic maps), cells with a repeated dof, rows too
+// long for a warp's shared memory, no memory for the records.
+void build_rows_plan(fe_form_s& f, cudaStream_t s) {
+  f.rows_plan.reset();
+  const int deg = degree_of(f.kind);
+  if (!deg || f.precision != FE_PREC_FP64 || f.V0 != f.V1 || f.V0->excluded || f.sp->parent || f.ffcx) return;
+  const fe_dofmap_s& V = *f.V0;
+  const fe_mesh_s& mesh = *f.mesh;
+  const int64_t C = V.num_cells, nR = V.num_blocks;
+  if (C == 0 || nR == 0 || V.k != dofs_of(deg) || C != mesh.num_cells || C * V.k > INT32_MAX || nR >= (1 << 30) ||
+      mesh.num_nodes > kStripVertex ||
+      capturing(s))
+    return;
+  int longest = 0;
+  for (int64_t r = 0; r < nR; ++r)
+    longest = std::max(longest, f.sp->host_row_ptr[r + 1] - f.sp->host_row_ptr[r]);
+  if (longest > 256) return;
+  try {
+    auto P = std::make_unique<fe_form_s::RowsPlan>();
+    DevBuf<int32_t> cnt(nR + 1), cursor(nR + 1), inc((size_t)C * V.k), row(nR), row_sorted(nR);
+    DevBuf<unsigned> kmask(nR), fail(1);
+    DevBuf<uint32_t> key(nR), key_sorted(nR);
+    DevBuf<int> kinds(3);
+    FE_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes(), s));
+    FE_CUDA(cudaMemsetAsync(kmask.p, 0, kmask.bytes(), s));
+    FE_CUDA(cudaMemsetAsync(fail.p, 0, fail.bytes(), s));
+    FE_CUDA(cudaMemsetAsync(kinds.p, 0, kinds.bytes(), s));
+    PlanArgs a{};
+    a.num_cells = C;
+    a.num_rows = nR;
+    a.k = V.k;
+    a.deg = deg;
+    a.geom = mesh.geom.p;
+    a.dofs = V.dofs.p;
+    a.pos = f.pos.p;
+    a.row_ptr = f.sp->row_ptr.p;
+    a.bs = V.bs;
+    a.inc_ptr = cnt.p;
+    a.inc = inc.p;
+    a.fail = fail.p;
+    k_rows_count<<<blocks_for(C, 128), 128, 0, s>>>(a, cnt.p, kmask.p);
+    FE_CUDA(cudaGetLastError());
+    k_rows_keys<<<blocks_for(nR, 256), 256, 0, s>>>(a, cnt.p, kmask.p, key.p, row.p, kinds.p);
+    FE_CUDA(cudaGetLastError());
+    exclusive_scan(cnt.p, nR + 1, s);
+    int hk[3];
+    unsigned bad = 0;
+    FE_CUDA(cudaMemcpyAsync(hk, kinds.p, sizeof(hk), cudaMemcpyDeviceToHost, s));
+    FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
+    FE_CUDA(cudaMemcpyAsync(cursor.p, cnt.p, cursor.bytes(), cudaMemcpyDeviceToDevice, s));
+    FE_CUDA(cudaStreamSynchronize(s));
+    if (bad) return;
+    k_rows_fill<<<blocks_for(C * V.k, 256), 256, 0, s>>>(a, cursor.p);
+    FE_CUDA(cudaGetLastError());
+    size_t tb = 0;
+    FE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key_sorted.p, row.p, row_sorted.p, (int)nR, 0, 32, s));
+    DevBuf<unsigned char> tmp(std::max<size_t>(1, tb));
+    FE_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key_sorted.p, row.p, row_sorted.p, (int)nR, 0, 32, s));
+    int64_t first = 0;
+    for (int kind = 0; kind < 3; ++kind) {
+      PartArgs p{};
+      p.kind = kind;
+      p.nrows = hk[kind];
+      p.ngroups = (hk[kind] + 31) / 32;
+      // few groups: their walks are shared by several warps, which shortens
+      // the chain of steps (us per call with 1 / 2 / 4: P1 n=12 15.7 / 9.7 /
+      // 6.8, n=32 (1,123 groups) 17.0 / 13.7 / 14.8, n=64 83 / 102 / 139; P2
+      // n=16 24 / 17 / 16, n=28 (763 groups) 48 / 42 / 46, n=60 320 / 358 / 415)
+      p.parts = 1;
+      if (kind == KIND_V) p.parts = p.ngroups <= 2 * f.ctx->num_sms ? 4 : (p.ngroups <= 10 * f.ctx->num_sms ? 2 : 1);
+      if (p.nrows == 0) continue;
+      build_part(a, p, P->part[kind], row_sorted.p + first, s);
+      first += p.nrows;
+    }
+    P->x4.alloc((size_t)std::max<int64_t>(1, mesh.num_nodes));
+    k_rows_pad_x<<<blocks_for(mesh.num_nodes, 256), 256, 0, s>>>(mesh.x.p, mesh.num_nodes, P->x4.p);
+    FE_CUDA(cudaGetLastError());
+    FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
+    FE_CUDA(cudaStreamSynchronize(s));  // the temporaries are freed on return
+    if (bad) return;
+    // the rows of a kind: a longer bound than needed for the others is fine
+    // for P1 and P2 edge rows are the shorter ones
+    P->part[KIND_V].stride = odd_at_least(longest);
+    int longest_e = 0;
+    if (hk[KIND_E]) {
+      std::vector<int32_t> he((size_t)hk[KIND_E]);
+      FE_CUDA(cudaMemcpy(he.data(), row_sorted.p + hk[KIND_V], he.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+      for (int32_t r : he) longest_e = std::max(longest_e, f.sp->host_row_ptr[r + 1] - f.sp->host_row_ptr[r]);
+    }
+    P->part[KIND_E].stride = odd_at_least(longest_e);
+    // at least four warps per SM, or the scatter is the better one
+    if (segment_bytes(P->part[KIND_V].stride) + kSmemCta > kSmemSm / 4 ||
+        segment_bytes(P->part[KIND_E].stride) + kSmemCta > kSmemSm / 4)
+      return;
+    if (deg == 1) raise_all<1>();
+    else raise_all<2>();
+    if (deg == 2) {
+      raise_smem(k_rows_e2<FE_COEFF_CONSTANT>);
+      raise_smem(k_rows_e2<FE_COEFF_DG0>);
+      raise_smem(k_rows_e2<FE_COEFF_P1>);
+    }
+    f.rows_plan = std::move(P);
+    const Coefficient& k = f.coeff[0];
+    if (k.kind == FE_COEFF_P1 && k.map) (void)vertex_numbered(f, *k.map, s);
+  } catch (const Error& e) {
+    if (e.code != FE_ERR_NOMEM) throw;
+    f.rows_plan.reset();
+  }
+}
+
+bool rows_supported(fe_form_s& f, const fe_bc_s* bc0, const fe_bc_s* bc1, cudaStream_t s) {
+  if (!f.rows_plan || f.precision != FE_PREC_FP64 || bc0 != bc1) return false;
+  const Coefficient& k = f.coeff[0];
+  if (k.kind == FE_COEFF_P1) {
+    if (!k.map || !vertex_numbered(f, *k.map, s)) return false;
+  } else if (k.kind != FE_COEFF_DG0 && k.kind != FE_COEFF_CONSTANT && k.kind >= 0) {
+    return false;
+  }
+  if (bc0 && bc0->row_flags.find(f.sp->id) == bc0->row_flags.end() && capturing(s)) return false;
+  return true;
+}
+
+namespace {
+// `beside`: the kernel before it in the stream is one of this call's
+template <typename K>
+void launch_beside(K kernel, unsigned grid, size_t smem, bool beside, const WalkArgs& a, cudaStream_t s) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(32);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = beside ? 1 : 0;
+  FE_CUDA(cudaLaunchKernelEx(&c, kernel, a));
+}
+
+template <int DEG, int COEF>
+void launch_parts(const fe_form_s& f, WalkArgs a, cudaStream_t s) {
+  const fe_form_s::RowsPlan& P = *f.rows_plan;
+  auto set = [&](const fe_form_s::RowsPlan::Part& p) {
+    a.ngroups = p.ngroups;
+    a.own = p.own.p;
+    a.steps = p.steps.p;
+    a.rec = p.rec.p;
+    a.rec1 = p.rec1.p;
+    a.cell = p.cell.p;
+    a.stride = p.stride;
+    a.gaps = p.gaps ? 1 : 0;
+  };
+  const auto& pv = P.part[KIND_V];
+  if (pv.ngroups) {
+    set(pv);
+    const unsigned grid = (unsigned)pv.ngroups;
+    const size_t seg = segment_bytes(pv.stride);
+    if (pv.parts == 4) k_rows_v<DEG, COEF, 4><<<grid, 128, 4 * seg, s>>>(a);
+    else if (pv.parts == 2) k_rows_v<DEG, COEF, 2><<<grid, 64, 2 * seg, s>>>(a);
+    else k_rows_v<DEG, COEF, 1><<<grid, 32, seg, s>>>(a);
+    FE_CUDA(cudaGetLastError());
+  }
+  const auto& pe = P.part[KIND_E];
+  if (DEG == 2 && pe.ngroups) {
+    set(pe);
+    launch_beside(k_rows_e2<COEF>, (unsigned)pe.ngroups, segment_bytes(pe.stride), pv.ngroups > 0, a, s);
+  }
+}
+}  // namespace
+
+void assemble_matrix_rows(fe_form_s& f, double* values, const fe_bc_s* bc, double diagonal, bool zero,
+                          cudaStream_t s) {
+  const fe_sparsity_s& sp = *f.sp;
+  WalkArgs a{};
+  a.x4 = f.rows_plan->x4.p;
+  const Coefficient& k = f.coeff[0];
+  a.coef = k.values;
+  a.coef_const = k.kind < 0 ? 1.0 : k.constant[0];
+  a.row_ptr = sp.row_ptr.p;
+  a.zero = zero ? 1 : 0;
+  a.values = values;
+  bool set_diag = false;
+  if (bc) {
+    // which rows a BC touches: once per (pattern, BC), as the diagonal slots of the zero pass
+    auto& F = bc->row_flags[sp.id];
+    if (!F) {
+      auto t = std::make_unique<fe_bc_s::RowFlags>();
+      t->flags.alloc((size_t)std::max<int64_t>(1, sp.num_rows));
+      t->mask.alloc((size_t)(sp.nnz / 32 + 1));
+      if (sp.nnz) k_rows_bc_mask<<<blocks_for(sp.nnz, 256), 256, 0, s>>>(sp.col.p, sp.nnz, bc->markers.p, t->mask.p);
+      k_rows_bc_flags<<<blocks_for(sp.num_rows, 256), 256, 0, s>>>(sp.row_ptr.p, sp.num_rows, bc->markers.p,
+                                                                   t->mask.p, t->flags.p);
+      FE_CUDA(cudaGetLastError());
+      FE_CUDA(cudaStreamSynchronize(s));  // calls on other streams may read them next
+      F = std::move(t);
+    }
+    a.flags = F->flags.p;
+    a.mask = F->mask.p;
+    // the marked rows are the owned listed ones: their diagonal goes with the rows
+    const bool owned = bc->markers_are_dofs && bc->n_owned == bc->n_bc;
+    a.diagonal = owned && zero ? diagonal : 0.0;
+    set_diag = !owned || !zero;
+  }
+  const int kind = k.kind < 0 ? FE_COEFF_CONSTANT : k.kind;
+  if (f.kind == FE_FORM_P1_STIFFNESS) {
+    if (kind == FE_COEFF_P1) launch_parts<1, FE_COEFF_P1>(f, a, s);
+    else if (kind == FE_COEFF_DG0) launch_parts<1, FE_COEFF_DG0>(f, a, s);
+    else launch_parts<1, FE_COEFF_CONSTANT>(f, a, s);
+  } else {
+    if (kind == FE_COEFF_P1) launch_parts<2, FE_COEFF_P1>(f, a, s);
+    else if (kind == FE_COEFF_DG0) launch_parts<2, FE_COEFF_DG0>(f, a, s);
+    else launch_parts<2, FE_COEFF_CONSTANT>(f, a, s);
+  }
+  if (set_diag) launch_set_diagonal(sp, *bc, diagonal, values, s);
+}
+
+}  // namespace fe

@@ -45,9 +45,10 @@ ASM_ZERO, ASM_DETERMINISTIC, ASM_ATOMIC, ASM_SORTED_SLOT, ASM_TILE, ASM_ROW_GATH
 ASM_FULL_SCATTER = 128
 ASM_GROUPED = 256
 ASM_COALESCED = 512
+ASM_ROW_WALK = 1024
 VARIANT_FLAGS = {"auto": 0, "deterministic": ASM_DETERMINISTIC, "atomic": ASM_ATOMIC, "sorted-slot": ASM_SORTED_SLOT,
                  "tile": ASM_TILE, "row-gather": ASM_ROW_GATHER, "block": ASM_BLOCK, "atomic-full": ASM_ATOMIC | ASM_FULL_SCATTER, "grouped": ASM_GROUPED,
-                 "coalesced": ASM_COALESCED}
+                 "coalesced": ASM_COALESCED, "row-walk": ASM_ROW_WALK}
 
 _SIGS = {
     "fe_last_error": (ctypes.c_char_p, []),

@@ -24,11 +24,13 @@ from .la import CUDAMatrix
 
 # matrix variants worth timing per form kind (all parity-tested)
 CANDIDATES = {
-    "P1_STIFFNESS": ("atomic", "block", "tile"),
-    "P2_STIFFNESS": ("atomic", "block", "grouped", "coalesced"),
+    "P1_STIFFNESS": ("atomic", "block", "tile", "row-walk"),
+    "P2_STIFFNESS": ("atomic", "block", "grouped", "coalesced", "row-walk"),
     "VP2_ELASTICITY": ("coalesced", "atomic", "atomic-full"),
     "P3_STIFFNESS": ("coalesced", "atomic"),  # coalesced: FP64 element tensors only (skipped for FP32)
 }
+# the row walk is timed from the sizes on where it is the engine's default
+ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536}
 # launch shapes of the atomic scatter timed per form kind: (cells per CTA,
 # byte maps staged in shared memory)
 LAUNCHES = {
@@ -66,7 +68,14 @@ class VariantTuner:
         sp = stream.cuda_stream
         best, best_ms, times = None, float("inf"), {}
         trials = []
+        # the row walk takes a field coefficient only when its dofmap is the
+        # mesh's vertex numbering, which the key does not tell: it is timed
+        # for constant and cellwise coefficients
+        field = any(getattr(getattr(c, "function_space", None), "degree", 0) for c in a._spec.coefficients)
         for v in CANDIDATES.get(a._spec.kind, ("atomic",)):
+            if v == "row-walk" and (field or a._spec.precision != "fp64"
+                                    or a._spec.mesh.num_cells < ROW_WALK_CELLS[a._spec.kind]):
+                continue
             shapes = LAUNCHES.get(a._spec.kind, ((0, 1),)) if v in ("atomic", "atomic-full") else ((0, 1),)
             trials += [(v, shape) for shape in shapes]
         for v, shape in trials:
