@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -86,7 +87,11 @@ struct fe_context_s {
   // between calls, instead of the default pool, which returns its memory at
   // every synchronise and maps it again on the next solve
   cudaMemPool_t scratch_pool = nullptr;
+  // page-locked records of the solvers, kept between calls (fe_pcg.cu)
+  std::mutex host_mutex;
+  std::vector<void*> host_records;
   ~fe_context_s() {
+    for (void* p : host_records) (void)cudaFreeHost(p);
     if (scratch_pool) (void)cudaMemPoolDestroy(scratch_pool);
   }
 };

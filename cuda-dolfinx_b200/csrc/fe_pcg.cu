@@ -6,8 +6,9 @@
 //   * SpMV with a sub-warp per row (width from the mean row length) fused
 //     with the p.Ap dot product;
 //   * x/r/z update fused with the r.z and r.r dot products;
-//   * dot products reduce per block into fixed slots, then one block sums the
-//     slots in a fixed order, so the iteration is bitwise reproducible;
+//   * dot products reduce per block into fixed slots, then one block (in the
+//     FP64 solver the last one of the same kernel) sums the slots in a fixed
+//     order, so the iteration is bitwise reproducible;
 //   * alpha/beta and the stopping test live on the device: every kernel
 //     returns immediately once `done` is set, so the host enqueues iterations
 //     in batches and synchronises once per batch.
@@ -27,7 +28,8 @@ constexpr int kThreads = 256;
 
 struct Scalars {
   double rz, rz_new, pAp, rr, bb, alpha, beta, tol2;
-  int iter, max_iter, done, pad;
+  int iter, max_iter, done;
+  unsigned arrived;  // blocks of the running kernel that have left their partial sums
 };
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {
@@ -144,6 +146,170 @@ __global__ void k_reduce(const double* __restrict__ part, int m, int stage, Scal
   }
 }
 
+// ---------------------------------------------------------------------------
+// One iteration of the FP64 solver in two kernels.  On matrices that fit the
+// L2 an iteration is a chain of launches: the five of before (SpMV, reduce,
+// update, reduce, p update) took 33.4 us at 91,125 rows and 2.5 M nonzeros
+// (28.8 us now; 26.9 -> 14.8 us at 4,913 rows):
+//   k_cg_spmv    p = z + beta p as it is read -- z and p stand in one 16-byte
+//                pair per row, so a column's gather is one load -- Ap = A p,
+//                then the last block sums p.Ap and sets alpha;
+//   k_cg_update  p again for the own row, x, r, z, then the last block sums
+//                r.z and r.r, sets beta and the stopping flag.
+// Each starts while the one before it drains (programmatic dependent launch)
+// and waits for it before reading what it wrote.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void start_after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
+// true in every thread of the block that finished last; its thread 0 has seen
+// all partial sums
+__device__ __forceinline__ bool last_block(Scalars* sc) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&sc->arrived, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
+__device__ __forceinline__ double sum_slots(const double* part, int m, double* sh) {
+  double v = 0.0;
+  for (int i = threadIdx.x; i < m; i += kThreads) v += __ldcg(part + i);
+  return block_sum(v, sh);
+}
+
+__device__ __forceinline__ void set_alpha(const double* part, Scalars* sc, double* sh) {
+  const double t = sum_slots(part, gridDim.x, sh);
+  if (threadIdx.x != 0) return;
+  sc->arrived = 0;
+  sc->pAp = t;
+  if (t == 0.0) sc->done = 1;
+  else sc->alpha = sc->rz / t;
+}
+
+// y = A p for R consecutive rows at a time: the block streams the rows'
+// nonzeros -- every thread on consecutive slots, eight columns, values and
+// gathered entries in flight at once, whatever the row bounds -- into shared
+// memory and then adds them up row by row, 256 / R lanes to a row.  What
+// bounds it is the gather: about 12 L1 wavefronts for 32 consecutive P2
+// columns (65 % of the L1's at 531,441 rows).
+constexpr int kStream = 2048;  // products in shared memory
+template <int R>
+__global__ void __launch_bounds__(kThreads) k_cg_spmv(int64_t n, const int32_t* __restrict__ rp,
+                                                      const int32_t* __restrict__ col,
+                                                      const double* __restrict__ val, const double2* zp,
+                                                      double* __restrict__ Ap, double* part, Scalars* sc) {
+  constexpr int LPR = kThreads / R;
+  __shared__ double prod[kStream];
+  __shared__ double sh[32];
+  __shared__ int32_t srp[R + 1];
+  start_after_previous();
+  if (sc->done) return;
+  const double beta = sc->beta;
+  auto p_at = [&](int64_t c) {
+    const double2 w = zp[c];  // (written by the kernel before: an ordinary load)
+    return fma(beta, w.y, w.x);
+  };
+  const int tid = threadIdx.x, row = tid / LPR, sub = tid % LPR;
+  double pap = 0.0;
+  for (int64_t r0 = blockIdx.x * (int64_t)R; r0 < n; r0 += (int64_t)gridDim.x * R) {
+    const int rows = (int)(n - r0 < R ? n - r0 : R);
+    __syncthreads();
+    for (int q = tid; q <= R; q += kThreads) srp[q] = __ldg(rp + r0 + (q < rows ? q : rows));
+    __syncthreads();
+    const int32_t lo = srp[row], hi = srp[row + 1], end = srp[R];
+    double acc = 0.0;
+    for (int32_t base = srp[0]; base < end; base += kStream) {
+      int32_t c[kStream / kThreads];
+      double v[kStream / kThreads];
+#pragma unroll
+      for (int q = 0; q < kStream / kThreads; ++q) {
+        const int32_t t = base + q * kThreads + tid;
+        c[q] = t < end ? __ldg(col + t) : 0;
+        v[q] = t < end ? __ldg(val + t) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < kStream / kThreads; ++q)
+        prod[q * kThreads + tid] = v[q] * p_at(c[q]);  // (past the end: never read)
+      __syncthreads();
+      const int32_t a = max(lo, base), b = min(hi, base + kStream);
+      for (int32_t t = a + sub; t < b; t += LPR) acc += prod[t - base];
+      __syncthreads();
+    }
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LPR);
+    if (row < rows && sub == 0) {
+      Ap[r0 + row] = acc;
+      pap += p_at(r0 + row) * acc;
+    }
+  }
+  pap = block_sum(pap, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = pap;
+  if (last_block(sc)) set_alpha(part, sc, sh);
+}
+
+__global__ void __launch_bounds__(kThreads) k_cg_update(int64_t n, double* __restrict__ x, double* __restrict__ r,
+                                                        double2* __restrict__ zp, const double* Ap,
+                                                        const double* __restrict__ dinv, double* part, Scalars* sc) {
+  __shared__ double sh[32];
+  start_after_previous();
+  if (sc->done) return;
+  const double alpha = sc->alpha, beta = sc->beta;
+  double rz = 0.0, rr = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads) {
+    const double2 q = zp[i];
+    const double pv = fma(beta, q.y, q.x);
+    x[i] += alpha * pv;
+    const double rv = r[i] - alpha * Ap[i];
+    r[i] = rv;
+    const double zv = dinv[i] * rv;
+    zp[i] = make_double2(zv, pv);
+    rz += rv * zv;
+    rr += rv * rv;
+  }
+  rz = block_sum(rz, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = rz;
+  rr = block_sum(rr, sh);
+  if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = rr;
+  if (!last_block(sc)) return;
+  const double rz_new = sum_slots(part, gridDim.x, sh), rr_new = sum_slots(part + gridDim.x, gridDim.x, sh);
+  if (threadIdx.x == 0) {
+    sc->arrived = 0;
+    sc->rz_new = rz_new;
+    sc->rr = rr_new;
+    sc->beta = rz_new / sc->rz;
+    sc->rz = rz_new;
+    sc->iter += 1;
+    if (rr_new <= sc->tol2 * sc->bb || sc->iter >= sc->max_iter) sc->done = 1;
+  }
+}
+
+template <typename K, typename... Args>
+void launch_chained(K kernel, unsigned grid, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(kThreads);
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  FE_CUDA(cudaLaunchKernelEx(&c, kernel, args...));
+}
+
+// z and p as the solver's pairs, from the separate vectors of k_init (p is
+// formed from them with beta = 0 in the first iteration)
+__global__ void __launch_bounds__(kThreads) k_cg_pairs(int64_t n, const double* __restrict__ z,
+                                                       double2* __restrict__ zp) {
+  for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads)
+    zp[i] = make_double2(z[i], 0.0);
+}
+
 template <int SUB>
 __global__ void __launch_bounds__(kThreads) k_spmv(int64_t n, const int32_t* __restrict__ rp,
                                                    const int32_t* __restrict__ col, const double* __restrict__ val,
@@ -243,47 +409,159 @@ struct StreamScratch {
   }
 };
 
+// host copies of the scalars, page-locked so that reading them back does not
+// stop the host: at most kKeptRecords pairs are kept between solves
+struct HostRecords {
+  fe_context_s& ctx;
+  Scalars* p = nullptr;  // two records
+  static constexpr size_t kKeptRecords = 16;
+  explicit HostRecords(fe_context_s& c) : ctx(c) {
+    {
+      std::lock_guard<std::mutex> lock(ctx.host_mutex);
+      if (!ctx.host_records.empty()) {
+        p = static_cast<Scalars*>(ctx.host_records.back());
+        ctx.host_records.pop_back();
+      }
+    }
+    if (!p) FE_CUDA(cudaMallocHost((void**)&p, 2 * sizeof(Scalars)));
+  }
+  HostRecords(const HostRecords&) = delete;
+  HostRecords& operator=(const HostRecords&) = delete;
+  ~HostRecords() {
+    {
+      std::lock_guard<std::mutex> lock(ctx.host_mutex);
+      if (ctx.host_records.size() < kKeptRecords) {
+        ctx.host_records.push_back(p);
+        return;
+      }
+    }
+    (void)cudaFreeHost(p);
+  }
+};
+
+struct Event {
+  cudaEvent_t e = nullptr;
+  Event() { FE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+  Event(const Event&) = delete;
+  Event& operator=(const Event&) = delete;
+  ~Event() { (void)cudaEventDestroy(e); }
+};
+
+// vectors of one solve
+struct CgVectors {
+  double *r, *Ap, *dinv, *part;
+  double2* zp;  // pairs, or for large matrices z and then p
+  Scalars* sc;
+  double* z() const { return reinterpret_cast<double*>(zp); }
+  double* p(int64_t n) const { return z() + n; }
+};
+
+// Up to this many nonzeros -- while a matrix and its vectors stay in the L2 and
+// launches count -- an iteration is the two kernels above; larger matrices keep
+// the five launches (row by row, no pairs: the gather is what counts there).
+// us an iteration on B200, two kernels / five: P2 n=8 (4,913 rows) 15 / 27,
+// n=22 (2.5 M nonzeros) 29 / 33, n=40 (14 M) 95 / 97; P1 n=22 15 / 22, n=64
+// (4 M) 40 / 43, n=110 (20 M) 159 / 155; P3 n=16 (5.5 M) 40 / 41; vector P2
+// n=8 21 / 27, n=20 (17 M) 111 / 73.
+constexpr int64_t kPairNonzeros = 6000000;
+
+// the launch shapes of both solvers: the row kernels (k_init, k_cg_spmv) wait
+// on dependent loads (row bounds -> columns and values -> gathered entries)
+// and run 8 CTAs per SM, the vector updates 4; each reduction sums the
+// partials of the launch that wrote them, so the partial sums are grouped
+// identically and fe_pcg_solve and fe_pcg_solve_noalloc agree bitwise
+template <int SUB>
+void cg_begin(const fe_sparsity_s& A, const double* val, const double* b, const double* x, const Scalars& h,
+              const CgVectors& v, unsigned grid, unsigned grid_rows, cudaStream_t s) {
+  const int64_t n = A.num_rows;
+  FE_CUDA(cudaMemcpyAsync(v.sc, &h, sizeof(h), cudaMemcpyHostToDevice, s));
+  const bool pairs = A.nnz <= kPairNonzeros;
+  // (for the pairs z goes through Ap, which is free until the first product; k_init's p is z)
+  k_init<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, A.diag.p, b, x, v.r,
+                                             pairs ? v.Ap : v.z(), pairs ? v.Ap : v.p(n), v.dinv, v.part);
+  k_reduce<<<1, 1024, 0, s>>>(v.part, grid_rows, 0, v.sc);
+  if (pairs) k_cg_pairs<<<grid, kThreads, 0, s>>>(n, v.Ap, v.zp);
+  FE_CUDA(cudaGetLastError());
+}
+
+
+template <int R>
+void cg_iteration(const fe_sparsity_s& A, const double* val, double* x, const CgVectors& v, unsigned grid,
+                  unsigned grid_rows, cudaStream_t s) {
+  const int64_t n = A.num_rows;
+  const unsigned gr = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_rows, (n + R - 1) / R));
+  const unsigned gu = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid, (n + kThreads - 1) / kThreads));
+  launch_chained(k_cg_spmv<R>, gr, s, n, (const int32_t*)A.row_ptr.p, (const int32_t*)A.col.p, val,
+                 (const double2*)v.zp, v.Ap, v.part, v.sc);
+  launch_chained(k_cg_update, gu, s, n, x, v.r, v.zp, (const double*)v.Ap, (const double*)v.dinv, v.part, v.sc);
+}
+
+// `count` iterations; rows of a stream tile: about 1,700 of its 2,048 products
+// at the mean row length of each class
+template <int SUB>
+void cg_batch(const fe_sparsity_s& A, const double* val, double* x, int count, const CgVectors& v, unsigned grid,
+              unsigned grid_rows, cudaStream_t s) {
+  const int64_t n = A.num_rows;
+  if (A.nnz > kPairNonzeros) {
+    double *z = v.z(), *p = v.p(n);
+    for (int q = 0; q < count; ++q) {
+      k_spmv<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, p, v.Ap, v.part, v.sc);
+      k_reduce<<<1, 1024, 0, s>>>(v.part, grid_rows, 1, v.sc);
+      k_update<<<grid, kThreads, 0, s>>>(n, x, v.r, z, p, v.Ap, v.dinv, v.part, v.sc);
+      k_reduce<<<1, 1024, 0, s>>>(v.part, grid, 2, v.sc);
+      k_update_p<<<grid, kThreads, 0, s>>>(n, z, p, v.sc);
+    }
+    FE_CUDA(cudaGetLastError());
+    return;
+  }
+  constexpr int R = SUB == 4 ? 256 : (SUB == 8 ? 128 : 64);
+  const double mean = n ? (double)A.nnz / (double)n : 0.0;
+  for (int q = 0; q < count; ++q) {
+    if (SUB < 32) cg_iteration<R>(A, val, x, v, grid, grid_rows, s);
+    else if (mean <= 60.0) cg_iteration<32>(A, val, x, v, grid, grid_rows, s);
+    else cg_iteration<16>(A, val, x, v, grid, grid_rows, s);
+  }
+}
+
 template <int SUB>
 void run(const fe_sparsity_s& A, const double* val, const double* b, double* x, double rtol, int max_iter,
          int* iterations, double* rel_res, cudaStream_t s) {
   const int64_t n = A.num_rows;
-  // the row kernels (k_init, k_spmv: 32 registers) wait on dependent loads
-  // (row bounds -> columns and values -> gathered entries): they run 8 CTAs
-  // per SM, the vector updates (40 registers) 4; each reduction sums the
-  // partials of the launch that wrote them
   const unsigned grid = (unsigned)(A.ctx->num_sms * 4);
   const unsigned grid_rows = (unsigned)(A.ctx->num_sms * 8);
   // stream-ordered scratch, released on every exit path (a launch or
   // synchronisation error inside the loop throws)
   StreamScratch buf(s, scratch_pool(*A.ctx));
-  double* r = buf.get<double>(n);
-  double* z = buf.get<double>(n);
-  double* p = buf.get<double>(n);
-  double* Ap = buf.get<double>(n);
-  double* dinv = buf.get<double>(n);
-  double* part = buf.get<double>(3 * (int64_t)grid_rows);
-  Scalars* sc = buf.get<Scalars>(1);
+  CgVectors v{};
+  v.r = buf.get<double>(n);
+  v.zp = buf.get<double2>(n);
+  v.Ap = buf.get<double>(n);
+  v.dinv = buf.get<double>(n);
+  v.part = buf.get<double>(3 * (int64_t)grid_rows);
+  v.sc = buf.get<Scalars>(1);
   Scalars h{};
   h.tol2 = rtol * rtol;
   h.max_iter = max_iter;
-  FE_CUDA(cudaMemcpyAsync(sc, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-  k_init<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, A.diag.p, b, x, r, z, p, dinv, part);
-  k_reduce<<<1, 1024, 0, s>>>(part, grid_rows, 0, sc);
-  FE_CUDA(cudaGetLastError());
-  const int batch = 16;
-  for (int it = 0;; it += batch) {
-    for (int q = 0; q < batch; ++q) {
-      k_spmv<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, p, Ap, part, sc);
-      k_reduce<<<1, 1024, 0, s>>>(part, grid_rows, 1, sc);
-      k_update<<<grid, kThreads, 0, s>>>(n, x, r, z, p, Ap, dinv, part, sc);
-      k_reduce<<<1, 1024, 0, s>>>(part, grid, 2, sc);
-      k_update_p<<<grid, kThreads, 0, s>>>(n, z, p, sc);
-    }
-    FE_CUDA(cudaGetLastError());
-    FE_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, s));
-    FE_CUDA(cudaStreamSynchronize(s));
-    if (h.done || it >= max_iter) break;
+  HostRecords rec(*A.ctx);
+  Event ev[2];
+  cg_begin<SUB>(A, val, b, x, h, v, grid, grid_rows, s);
+  // short iterations: a batch is always queued behind the one whose outcome
+  // is waited for, so the device does not idle while the host looks at it
+  const bool ahead = A.nnz <= kPairNonzeros;
+  const int batch = ahead ? 8 : 16;
+  int last = 0;
+  for (int k = 0;; ++k) {
+    cg_batch<SUB>(A, val, x, batch, v, grid, grid_rows, s);
+    FE_CUDA(cudaMemcpyAsync(rec.p + (k & 1), v.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
+    FE_CUDA(cudaEventRecord(ev[k & 1].e, s));
+    last = k;
+    const int seen = ahead ? k - 1 : k;
+    if (seen < 0) continue;
+    FE_CUDA(cudaEventSynchronize(ev[seen & 1].e));
+    if (rec.p[seen & 1].done || (int64_t)seen * batch >= max_iter) break;
   }
+  FE_CUDA(cudaEventSynchronize(ev[last & 1].e));  // the record is written until then
+  h = rec.p[last & 1];
   buf.release();
   *iterations = h.iter;
   *rel_res = h.bb > 0 ? sqrt(h.rr / h.bb) : 0.0;
@@ -344,7 +622,7 @@ constexpr int kNoAllocMaxGrid = 2048;                   // reduction slots per d
 constexpr int64_t kNoAllocScalarWords = 16;            // room for one Scalars record (in doubles)
 static_assert(sizeof(Scalars) <= kNoAllocScalarWords * sizeof(double), "Scalars record does not fit");
 
-// r, z, p, Ap, dinv (kNoAllocMaxRows each), 3 x kNoAllocMaxGrid partial sums, one Scalars record:
+// zp (pairs, or z and p), r, Ap, dinv (kNoAllocMaxRows each), 3 x kNoAllocMaxGrid partial sums, one Scalars record:
 // 5 * 262,144 * 8 B + 3 * 2048 * 8 B + 128 B = 10.5 MB held by every device that loads the library.
 static __device__ __align__(256) double g_pcg_scratch[5 * kNoAllocMaxRows + 3 * kNoAllocMaxGrid +
                                                       kNoAllocScalarWords];
@@ -368,41 +646,27 @@ double* scratch_address(int device) {
 template <int SUB>
 void run_noalloc(const fe_sparsity_s& A, const double* val, const double* b, double* x, double rtol, int max_iter,
                  int* iterations, double* rel_res, double* scratch, cudaStream_t s) {
-  const int64_t n = A.num_rows;
-  // the launch shapes of fe_pcg_solve (8 CTAs per SM for the row kernels, 4
-  // for the vector updates), so the partial sums are grouped identically and
-  // the two solvers give bitwise-equal results on the same GPU
   const unsigned grid = (unsigned)std::min(A.ctx->num_sms * 4, kNoAllocMaxGrid);
   const unsigned grid_rows = (unsigned)std::min(A.ctx->num_sms * 8, kNoAllocMaxGrid);
-  double* r = scratch;
-  double* z = r + kNoAllocMaxRows;
-  double* p = z + kNoAllocMaxRows;
-  double* Ap = p + kNoAllocMaxRows;
-  double* dinv = Ap + kNoAllocMaxRows;
-  double* part = dinv + kNoAllocMaxRows;
-  Scalars* sc = reinterpret_cast<Scalars*>(part + 3 * kNoAllocMaxGrid);
+  CgVectors v{};
+  v.zp = reinterpret_cast<double2*>(scratch);
+  v.r = scratch + 2 * kNoAllocMaxRows;
+  v.Ap = v.r + kNoAllocMaxRows;
+  v.dinv = v.Ap + kNoAllocMaxRows;
+  v.part = v.dinv + kNoAllocMaxRows;
+  v.sc = reinterpret_cast<Scalars*>(v.part + 3 * kNoAllocMaxGrid);
   // Every scratch word a kernel reads is written earlier in the same call:
-  // k_init writes r, z, p, dinv for all n rows, k_spmv writes Ap before
-  // k_update reads it, partial sums are written before each reduction, and
-  // the Scalars record is re-initialised here.
+  // k_init writes r, z and dinv for all n rows and k_cg_pairs the pairs,
+  // k_cg_spmv writes Ap before k_cg_update reads it, partial sums are written
+  // before each reduction, and the Scalars record is re-initialised here.
   Scalars h{};
   h.tol2 = rtol * rtol;
   h.max_iter = max_iter;
-  FE_CUDA(cudaMemcpyAsync(sc, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-  k_init<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, A.diag.p, b, x, r, z, p, dinv, part);
-  k_reduce<<<1, 1024, 0, s>>>(part, grid_rows, 0, sc);
-  FE_CUDA(cudaGetLastError());
+  cg_begin<SUB>(A, val, b, x, h, v, grid, grid_rows, s);
   const int batch = 16;
   for (int it = 0;; it += batch) {
-    for (int q = 0; q < batch; ++q) {
-      k_spmv<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, p, Ap, part, sc);
-      k_reduce<<<1, 1024, 0, s>>>(part, grid_rows, 1, sc);
-      k_update<<<grid, kThreads, 0, s>>>(n, x, r, z, p, Ap, dinv, part, sc);
-      k_reduce<<<1, 1024, 0, s>>>(part, grid, 2, sc);
-      k_update_p<<<grid, kThreads, 0, s>>>(n, z, p, sc);
-    }
-    FE_CUDA(cudaGetLastError());
-    FE_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, s));
+    cg_batch<SUB>(A, val, x, batch, v, grid, grid_rows, s);
+    FE_CUDA(cudaMemcpyAsync(&h, v.sc, sizeof(h), cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaStreamSynchronize(s));
     if (h.done || it >= max_iter) break;
   }
