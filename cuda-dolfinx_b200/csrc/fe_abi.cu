@@ -983,7 +983,7 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
     if (flags & FE_ASM_ROW_WALK) {
       if (!a->rows_plan && !view) build_rows_plan(*a, st);
       FE_REQUIRE(!view && rows_supported(*a, bc0, bc1, st),
-                 "the row walk supports FP64 P1/P2 stiffness with one space and one set of BCs, on conforming cells");
+                 "the row walk supports FP64 P1/P2/P3 stiffness with one space and one set of BCs, on conforming cells");
     }
     if (!(flags & (FE_ASM_ATOMIC | FE_ASM_FULL_SCATTER | FE_ASM_BLOCK | FE_ASM_COALESCED | FE_ASM_GROUPED)) && !view &&
         rows_supported(*a, bc0, bc1, st)) {

@@ -1726,6 +1726,97 @@ __device__ __forceinline__ void p2_mass_p1coef(const T* cq, Emit&& emit) {
   emit(9, 9, (fma(cq[2], T(0x1.a01a01a01a01ap-10), cq[0] * T(0x1.3813813813814p-8)) + fma(cq[3], T(0x1.a01a01a01a01ap-10), cq[1] * T(0x1.3813813813814p-8))));
 }
 
+// P3 stiffness row of vertex a: g[q] = k |det J| times the products of the gradients
+// ab, ac, ad, bc, bd, cd; emit(column, value), columns a, b, c, d, ab ba ac ca ad da bc cb bd db cd dc (xy: on edge xy near x), abc abd acd bcd.
+__constant__ double kP3RowV[9] = {
+    -0x1.e79e79e79e79ep-5, 0x1.7297297297297p-7, 0x1.8af8af8af8af9p-4, 0x1.1d41d41d41d42p-5, -0x1.8af8af8af8af9p-5, -0x1.b6db6db6db6dbp-7,
+    0x1.b6db6db6db6dbp-7, -0x1.0750750750750p-5, 0x1.0750750750750p-5,
+};
+template <typename Emit>
+__device__ __forceinline__ void p3_row_v(const double* g, Emit&& emit) {
+  emit(0, fma(g[2], kP3RowV[0], g[0] * kP3RowV[0]) + g[1] * kP3RowV[0]);
+  emit(1, g[0] * kP3RowV[1]);
+  emit(2, g[1] * kP3RowV[1]);
+  emit(3, g[2] * kP3RowV[1]);
+  emit(4, fma(g[2], kP3RowV[3], g[0] * kP3RowV[2]) + g[1] * kP3RowV[3]);
+  emit(5, fma(g[2], kP3RowV[5], g[0] * kP3RowV[4]) + g[1] * kP3RowV[5]);
+  emit(6, fma(g[2], kP3RowV[3], g[0] * kP3RowV[3]) + g[1] * kP3RowV[2]);
+  emit(7, fma(g[2], kP3RowV[5], g[0] * kP3RowV[5]) + g[1] * kP3RowV[4]);
+  emit(8, fma(g[2], kP3RowV[2], g[0] * kP3RowV[3]) + g[1] * kP3RowV[3]);
+  emit(9, fma(g[2], kP3RowV[4], g[0] * kP3RowV[5]) + g[1] * kP3RowV[5]);
+  emit(10, g[0] * kP3RowV[6] + g[1] * kP3RowV[6]);
+  emit(11, g[0] * kP3RowV[6] + g[1] * kP3RowV[6]);
+  emit(12, g[0] * kP3RowV[6] + g[2] * kP3RowV[6]);
+  emit(13, g[0] * kP3RowV[6] + g[2] * kP3RowV[6]);
+  emit(14, g[1] * kP3RowV[6] + g[2] * kP3RowV[6]);
+  emit(15, g[1] * kP3RowV[6] + g[2] * kP3RowV[6]);
+  emit(16, fma(g[2], kP3RowV[7], g[0] * kP3RowV[4]) + g[1] * kP3RowV[4]);
+  emit(17, fma(g[2], kP3RowV[4], g[0] * kP3RowV[4]) + g[1] * kP3RowV[7]);
+  emit(18, fma(g[2], kP3RowV[4], g[0] * kP3RowV[7]) + g[1] * kP3RowV[4]);
+  emit(19, fma(g[2], kP3RowV[8], g[0] * kP3RowV[8]) + g[1] * kP3RowV[8]);
+}
+
+// P3 stiffness row of the node of edge ab near a: g[q] = k |det J| times the products of the gradients
+// ab, ac, ad, bc, bd, cd; emit(column, value), columns a, b, ab, ba, c, ac ca bc cb, abc, d, ad da bd db, abd, cd dc, acd, bcd.
+__constant__ double kP3RowE[17] = {
+    0x1.8af8af8af8af9p-4, 0x1.1d41d41d41d42p-5, -0x1.8af8af8af8af9p-5, -0x1.b6db6db6db6dbp-7, -0x1.edb6db6db6db7p-3, -0x1.8af8af8af8af9p-3,
+    0x1.8af8af8af8af9p-3, 0x1.283a83a83a83bp-4, 0x1.b6db6db6db6dbp-7, -0x1.8af8af8af8af9p-6, -0x1.edb6db6db6db7p-4, -0x1.283a83a83a83bp-4,
+    0x1.8af8af8af8af9p-6, 0x1.8af8af8af8af9p-5, 0x1.283a83a83a83bp-2, -0x1.8af8af8af8af9p-4, 0x1.283a83a83a83bp-3,
+};
+template <typename Emit>
+__device__ __forceinline__ void p3_row_e(const double* g, Emit&& emit) {
+  emit(0, fma(g[2], kP3RowE[1], g[0] * kP3RowE[0]) + g[1] * kP3RowE[1]);
+  emit(1, fma(g[4], kP3RowE[3], g[0] * kP3RowE[2]) + g[3] * kP3RowE[3]);
+  emit(2, fma(g[4], kP3RowE[5], fma(g[2], kP3RowE[4], g[0] * kP3RowE[4])) + fma(g[3], kP3RowE[5], g[1] * kP3RowE[4]));
+  emit(3, fma(g[4], kP3RowE[7], fma(g[2], kP3RowE[7], g[0] * kP3RowE[6])) + fma(g[3], kP3RowE[7], g[1] * kP3RowE[7]));
+  emit(4, g[1] * kP3RowE[8] + g[3] * kP3RowE[8]);
+  emit(5, fma(g[2], kP3RowE[10], g[0] * kP3RowE[9]) + fma(g[3], kP3RowE[6], g[1] * kP3RowE[9]));
+  emit(6, fma(g[3], kP3RowE[11], g[1] * kP3RowE[9]) + g[2] * kP3RowE[12]);
+  emit(7, fma(g[4], kP3RowE[12], g[0] * kP3RowE[9]) + g[1] * kP3RowE[11]);
+  emit(8, g[1] * kP3RowE[2] + g[4] * kP3RowE[12]);
+  emit(9, fma(g[2], kP3RowE[13], g[0] * kP3RowE[13]) + fma(g[4], kP3RowE[15], g[1] * kP3RowE[14]));
+  emit(10, g[2] * kP3RowE[8] + g[4] * kP3RowE[8]);
+  emit(11, fma(g[2], kP3RowE[9], g[0] * kP3RowE[9]) + fma(g[4], kP3RowE[6], g[1] * kP3RowE[10]));
+  emit(12, fma(g[4], kP3RowE[11], g[1] * kP3RowE[12]) + g[2] * kP3RowE[9]);
+  emit(13, fma(g[3], kP3RowE[12], g[0] * kP3RowE[9]) + g[2] * kP3RowE[11]);
+  emit(14, g[2] * kP3RowE[2] + g[3] * kP3RowE[12]);
+  emit(15, fma(g[2], kP3RowE[14], g[0] * kP3RowE[13]) + fma(g[3], kP3RowE[15], g[1] * kP3RowE[13]));
+  emit(16, fma(g[3], kP3RowE[9], g[1] * kP3RowE[9]) + fma(g[4], kP3RowE[9], g[2] * kP3RowE[9]));
+  emit(17, fma(g[3], kP3RowE[9], g[1] * kP3RowE[9]) + fma(g[4], kP3RowE[9], g[2] * kP3RowE[9]));
+  emit(18, fma(g[3], kP3RowE[0], g[1] * kP3RowE[16]) + fma(g[4], kP3RowE[0], g[2] * kP3RowE[16]));
+  emit(19, g[1] * kP3RowE[2] + g[2] * kP3RowE[2]);
+}
+
+// P3 stiffness row of the node of face abc: g[q] = k |det J| times the products of the gradients
+// ab, ac, ad, bc, bd, cd; emit(column, value), columns a, b, c, ab ba ac ca bc cb, abc, d, ad da bd db cd dc, abd, acd, bcd.
+__constant__ double kP3RowF[11] = {
+    -0x1.8af8af8af8af9p-5, -0x1.0750750750750p-5, 0x1.8af8af8af8af9p-5, 0x1.283a83a83a83bp-2, -0x1.8af8af8af8af9p-4, -0x1.283a83a83a83bp-1,
+    0x1.0750750750750p-5, 0x1.283a83a83a83bp-3, 0x1.8af8af8af8af9p-4, -0x1.283a83a83a83bp-2, 0x1.283a83a83a83bp-1,
+};
+template <typename Emit>
+__device__ __forceinline__ void p3_row_f(const double* g, Emit&& emit) {
+  emit(0, fma(g[2], kP3RowF[1], g[0] * kP3RowF[0]) + g[1] * kP3RowF[0]);
+  emit(1, fma(g[4], kP3RowF[1], g[0] * kP3RowF[0]) + g[3] * kP3RowF[0]);
+  emit(2, fma(g[5], kP3RowF[1], g[1] * kP3RowF[0]) + g[3] * kP3RowF[0]);
+  emit(3, fma(g[2], kP3RowF[2], g[0] * kP3RowF[2]) + fma(g[4], kP3RowF[4], g[1] * kP3RowF[3]));
+  emit(4, fma(g[3], kP3RowF[3], g[0] * kP3RowF[2]) + fma(g[4], kP3RowF[2], g[2] * kP3RowF[4]));
+  emit(5, fma(g[2], kP3RowF[2], g[0] * kP3RowF[3]) + fma(g[5], kP3RowF[4], g[1] * kP3RowF[2]));
+  emit(6, fma(g[3], kP3RowF[3], g[1] * kP3RowF[2]) + fma(g[5], kP3RowF[2], g[2] * kP3RowF[4]));
+  emit(7, fma(g[4], kP3RowF[2], g[0] * kP3RowF[3]) + fma(g[5], kP3RowF[4], g[3] * kP3RowF[2]));
+  emit(8, fma(g[4], kP3RowF[4], g[1] * kP3RowF[3]) + fma(g[5], kP3RowF[2], g[3] * kP3RowF[2]));
+  emit(9, fma(g[4], kP3RowF[5], fma(g[2], kP3RowF[5], g[0] * kP3RowF[5])) + fma(g[5], kP3RowF[5], fma(g[3], kP3RowF[5], g[1] * kP3RowF[5])));
+  emit(10, fma(g[5], kP3RowF[6], g[2] * kP3RowF[6]) + g[4] * kP3RowF[6]);
+  emit(11, fma(g[4], kP3RowF[8], g[0] * kP3RowF[7]) + fma(g[5], kP3RowF[8], g[1] * kP3RowF[7]));
+  emit(12, g[4] * kP3RowF[0] + g[5] * kP3RowF[0]);
+  emit(13, fma(g[3], kP3RowF[7], g[0] * kP3RowF[7]) + fma(g[5], kP3RowF[8], g[2] * kP3RowF[8]));
+  emit(14, g[2] * kP3RowF[0] + g[5] * kP3RowF[0]);
+  emit(15, fma(g[3], kP3RowF[7], g[1] * kP3RowF[7]) + fma(g[4], kP3RowF[8], g[2] * kP3RowF[8]));
+  emit(16, g[2] * kP3RowF[0] + g[4] * kP3RowF[0]);
+  emit(17, g[0] * kP3RowF[9] + g[5] * kP3RowF[10]);
+  emit(18, g[1] * kP3RowF[9] + g[4] * kP3RowF[10]);
+  emit(19, g[2] * kP3RowF[10] + g[3] * kP3RowF[9]);
+}
+
 #ifdef FE_FACET_TABLES
 // cell-local dofs on each facet (P1)
 static __constant__ int kFacetDofsP1[4][3] = {{1, 2, 3}, {0, 2, 3}, {0, 1, 3}, {0, 1, 2}};

@@ -311,6 +311,8 @@ struct fe_form_s::RowsPlan {
     fe::DevBuf<int4> own;             // [groups*32] row (-1: none), its vertices, the slots of its own columns
     fe::DevBuf<int32_t> steps;        // [groups+1] prefix sums of the groups' longest walks
     fe::DevBuf<uint4> rec;            // records: vertices with marks, slot bytes
+    fe::DevBuf<uint4> rec2;           // P3: the rest of the records
+    fe::DevBuf<int4> own2;            // P3 face rows: the slots of their own columns
     fe::DevBuf<uint2> rec1;           // P1 records
     fe::DevBuf<int32_t> cell;         // cell of each record
   };

@@ -453,7 +453,7 @@ struct CgVectors {
   double2* zp;  // pairs, or for large matrices z and then p
   Scalars* sc;
   double* z() const { return reinterpret_cast<double*>(zp); }
-  double* p(int64_t n) const { return z() + n; }
+  double* p(int64_t n) const { return z() + (n + 31) / 32 * 32; }
 };
 
 // Up to this many nonzeros -- while a matrix and its vectors stay in the L2 and
@@ -534,7 +534,7 @@ void run(const fe_sparsity_s& A, const double* val, const double* b, double* x, 
   StreamScratch buf(s, scratch_pool(*A.ctx));
   CgVectors v{};
   v.r = buf.get<double>(n);
-  v.zp = buf.get<double2>(n);
+  v.zp = buf.get<double2>(n + 32);
   v.Ap = buf.get<double>(n);
   v.dinv = buf.get<double>(n);
   v.part = buf.get<double>(3 * (int64_t)grid_rows);

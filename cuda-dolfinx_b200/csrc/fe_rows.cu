@@ -34,6 +34,7 @@
 #include <cub/cub.cuh>
 #include <memory>
 
+#include "fe_element_code.cuh"
 #include "fe_internal.h"
 
 namespace fe {
@@ -183,6 +184,8 @@ struct PartArgs {
   int4* own;             // [ngroups*32]
   int32_t* steps;        // [ngroups+1] records of the longest row of each group, then their prefix sum
   uint4* rec;
+  uint4* rec2;           // P3: the rest of the records
+  int4* own2;            // face rows: their own slots
   uint2* rec1;           // P1 records
   int32_t* cell;
   unsigned* gaps;        // set when a row has slots that no cell adds to
@@ -332,13 +335,24 @@ __global__ void k_rows_head(const PlanArgs a, const PartArgs p) {
       int i, g[4], o[4];
       load_cell(a, inc[q], c, i, g);
       row_order(a.deg, i, g, o);
-      const uint32_t w = own_slots(a.deg, p.kind, a.pos + (c * a.k + i) * a.k, i, o);
+      const uint32_t w =
+          p.kind == KIND_F ? 0u : own_slots(a.deg, p.kind, a.pos + (c * a.k + i) * a.k, i, o);
       const int va = g[o[0]], vb = p.kind == KIND_V ? -1 : g[o[1]];
       if (q == 0) {
         own.y = va;
         own.z = vb;
-        own.w = (int)w;
-      } else if (p.kind != KIND_F && (own.y != va || own.z != vb || (uint32_t)own.w != w)) {
+        own.w = p.kind == KIND_F ? g[o[2]] : (int)w;
+        if (p.kind == KIND_F) {
+          // a, b, c, ab ba ac ca bc cb, the face
+          const uint8_t* b = a.pos + (c * a.k + i) * a.k;
+          auto B = [&](int j) -> uint32_t { return b[j]; };
+          p.own2[t] = make_int4(
+              (int)(B(o[0]) | (B(o[1]) << 8) | (B(o[2]) << 16) | (B(p3_edge(o[0], o[1])) << 24)),
+              (int)(B(p3_edge(o[1], o[0])) | (B(p3_edge(o[0], o[2])) << 8) | (B(p3_edge(o[2], o[0])) << 16) |
+                    (B(p3_edge(o[1], o[2])) << 24)),
+              (int)(B(p3_edge(o[2], o[1])) | (B(i) << 8)), 0);
+        }
+      } else if (own.y != va || own.z != vb || (uint32_t)own.w != (p.kind == KIND_F ? (uint32_t)g[o[2]] : w)) {
         *a.fail = 1u;  // one dof, several vertices or edges
       }
     }
@@ -403,6 +417,7 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
         p.cell[at] = 0;
         if (a.deg == 1) p.rec1[at] = make_uint2(kStripLoad, 0u);
         else p.rec[at] = make_uint4(kStripLoad, 0u, 0u, 0u);
+        if (a.deg == 3) p.rec2[at] = make_uint4(0u, 0u, 0u, 0u);
       }
     };
     if (n > 0 && n <= kMaxStar)
@@ -413,7 +428,7 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
           s = 0;
         }
         const int64_t at = (s0 + part * np + s++) * 32 + lane;
-        uint4 w = make_uint4((uint32_t)r3 | flags, 0u, 0u, 0u);
+        uint4 w = make_uint4((uint32_t)r3 | flags, 0u, 0u, 0u), w2 = make_uint4(0u, 0u, 0u, 0u);
         p.cell[at] = 0;
         if (t >= 0) {
           int64_t c;
@@ -436,10 +451,18 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
             w.z = B(p2_edge(i, lq)) | (B(p2_edge(i, lr)) << 8) | (B(p2_edge(lp, lq)) << 16) |
                   (B(p2_edge(lp, lr)) << 24);
             w.w = B(p2_edge(lq, lr));
+          } else if (a.deg == 3) {
+            auto E = [&](int x, int y) { return B(p3_edge(x, y)); };
+            w.y |= E(i, lp) << 24;
+            w.z = E(lp, i) | (E(i, lq) << 8) | (E(lq, i) << 16) | (E(i, lr) << 24);
+            w.w = E(lr, i) | (E(lp, lq) << 8) | (E(lq, lp) << 16) | (E(lp, lr) << 24);
+            w2.x = E(lr, lp) | (E(lq, lr) << 8) | (E(lr, lq) << 16) | (B(16 + lr) << 24);
+            w2.y = B(16 + lq) | (B(16 + lp) << 8) | (B(16 + i) << 16);
           }
         }
         if (a.deg == 1) p.rec1[at] = make_uint2(w.x, w.y);
         else p.rec[at] = w;
+        if (a.deg == 3) p.rec2[at] = w2;
       });
     while (at_part < p.parts) {
       rest();
@@ -452,6 +475,7 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
     if (s >= n) {
       p.cell[at] = 0;
       p.rec[at] = make_uint4(kAll, kAll, 0u, 0u);
+      if (a.deg == 3) p.rec2[at] = make_uint4(0u, 0u, 0u, 0u);
       continue;
     }
     int64_t c;
@@ -537,7 +561,29 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
     auto B = [&](int j) -> uint32_t { return q[j]; };
     for (int j = 0; j < a.k; ++j) mark(B(j));
     p.cell[at] = (int32_t)c;
-    {
+    if (a.deg == 3) {
+      // slots: the six of vertex c (c, ac ca bc cb, abc), the six of d, then cd dc acd bcd
+      auto E = [&](int x, int y) { return B(p3_edge(o[x], o[y])); };
+      uint4 w, w2;
+      w.x = (uint32_t)g[o[2]];
+      w.y = (uint32_t)g[o[3]];
+      w.z = B(o[2]) | (E(0, 2) << 8) | (E(2, 0) << 16) | (E(1, 2) << 24);
+      w.w = E(2, 1) | (B(16 + o[3]) << 8) | (B(o[3]) << 16) | (E(0, 3) << 24);
+      w2.x = E(3, 0) | (E(1, 3) << 8) | (E(3, 1) << 16) | (B(16 + o[2]) << 24);
+      w2.y = E(2, 3) | (E(3, 2) << 8) | (B(16 + o[1]) << 16) | (B(16 + o[0]) << 24);
+      w2.z = flags;
+      w2.w = 0u;
+      p.rec[at] = w;
+      p.rec2[at] = w2;
+      const uint32_t cs[6] = {w.z & 0xffu, (w.z >> 8) & 0xffu, (w.z >> 16) & 0xffu,
+                              w.z >> 24,   w.w & 0xffu,        (w.w >> 8) & 0xffu};
+      const uint32_t ds[6] = {(w.w >> 16) & 0xffu, w.w >> 24,           w2.x & 0xffu,
+                              (w2.x >> 8) & 0xffu, (w2.x >> 16) & 0xffu, w2.x >> 24};
+      for (int q2 = 0; q2 < 6; ++q2) write(cs[q2]);
+      for (int q2 = 0; q2 < 4; ++q2) write((w2.y >> (8 * q2)) & 0xffu);
+      if ((flags & kFanEnd) && !(flags & kFanClosed))
+        for (int q2 = 0; q2 < 6; ++q2) write(ds[q2]);
+    } else {
       uint4 w;
       w.x = (uint32_t)g[o[2]];
       w.y = (uint32_t)g[o[3]];
@@ -557,6 +603,31 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
         write((w.w >> 8) & 0xffu);
       }
     }
+  }
+  for (int s = 0; s < (p.kind == KIND_F ? ns : 0); ++s) {
+    const int64_t at = (s0 + s) * 32 + lane;
+    uint4 w = make_uint4(kAll, 0u, 0u, 0u);
+    p.cell[at] = 0;
+    if (s < n) {
+      int64_t c;
+      int i, g[4], o[4];
+      load_cell(a, inc[s], c, i, g);
+      row_order(a.deg, i, g, o);
+      const uint8_t* q = a.pos + (c * a.k + i) * a.k;
+      auto B = [&](int j) -> uint32_t { return q[j]; };
+      auto E = [&](int x, int y) { return B(p3_edge(o[x], o[y])); };
+      for (int j = 0; j < a.k; ++j) mark(B(j));
+      // slots: d, ad da bd db cd dc, abd acd bcd
+      w.x = (uint32_t)g[o[3]];
+      w.y = B(o[3]) | (E(0, 3) << 8) | (E(3, 0) << 16) | (E(1, 3) << 24);
+      w.z = E(3, 1) | (E(2, 3) << 8) | (E(3, 2) << 16) | (B(16 + o[2]) << 24);
+      w.w = B(16 + o[1]) | (B(16 + o[0]) << 8);
+      p.cell[at] = (int32_t)c;
+      for (int q2 = 0; q2 < 4; ++q2) write((w.y >> (8 * q2)) & 0xffu);
+      for (int q2 = 0; q2 < 4; ++q2) write((w.z >> (8 * q2)) & 0xffu);
+      for (int q2 = 0; q2 < 2; ++q2) write((w.w >> (8 * q2)) & 0xffu);
+    }
+    p.rec[at] = w;
   }
   if (r >= 0) {
     int covered = 0;
@@ -608,6 +679,8 @@ struct WalkArgs {
   const int4* __restrict__ own;
   const int32_t* __restrict__ steps;
   const uint4* __restrict__ rec;
+  const uint4* __restrict__ rec2;
+  const int4* __restrict__ own2;
   const uint2* __restrict__ rec1;
   const int32_t* __restrict__ cell;
   const double4* __restrict__ x4;
@@ -691,22 +764,23 @@ __device__ __forceinline__ void store_rows(const WalkArgs& a, double* acc, const
     }
   }
   __syncwarp();
-  const int len0 = __shfl_sync(kAll, at.len, 0);
-  if (a.zero && len0 > 0 && __all_sync(kAll, at.len == len0)) {
-    // 32 rows of one length: the lanes go through their entries without a gap
-    const int jump = 32 / len0, rest = 32 - jump * len0, end = first + count;
+  const int len0 = __shfl_sync(kAll, at.len, first);
+  if (a.zero && len0 > 0 && __all_sync(kAll, at.len == len0 || !((mine >> lane) & 1u))) {
+    // rows of one length: the lanes go through their entries without a gap
+    const int jump = 32 / len0, rest = 32 - jump * len0, end = (first + count) * len0, pad = a.stride - len0;
+    // entry t of the group stands at value index t + delta of its row
+    const int delta = at.lo - lane * len0;
     int rr = lane / len0, s = lane - rr * len0;
     rr += first;
+    const double* from = acc + first * len0 + lane;
 #pragma unroll 4
-    for (int it = 0; it < count * len0; it += 32) {
-      const int rlo = __shfl_sync(kAll, at.lo, rr);
-      if (rr < end) a.values[rlo + s] = acc[rr * a.stride + s];
-      rr += jump;
+    for (int t = first * len0 + lane; t < end + lane; t += 32, from += 32) {
+      const int to = t + __shfl_sync(kAll, delta, rr);
+      if (t < end) a.values[to] = from[rr * pad];
       s += rest;
-      if (s >= len0) {
-        s -= len0;
-        ++rr;
-      }
+      const bool wrap = s >= len0;
+      if (wrap) s -= len0;
+      rr += wrap ? jump + 1 : jump;
     }
     return;
   }
@@ -726,7 +800,7 @@ __device__ __forceinline__ void store_rows(const WalkArgs& a, double* acc, const
 // (P2 n=96: 1.15 ms against 1.22 ms with CTAs of two and four warps).
 // CTAs per SM to fit in registers (fewer registers spill, more leave too few
 // warps):
-constexpr int kMinV1 = 20, kMinV2 = 13, kMinE = 20;
+constexpr int kMinV1 = 20, kMinV2 = 13, kMinE = 20, kMinE3 = 16, kMinF3 = 20;
 
 // The kernels of one call write different rows: the later one starts while
 // the earlier one runs (programmatic dependent launch) and ends after it, so
@@ -1021,6 +1095,253 @@ __global__ void __launch_bounds__(32, kMinE) k_rows_e2(const WalkArgs a) {
   end_after_previous();
 }
 
+// ---------------------------------------------------------------------------
+// P3 (constant or cellwise k): the same walks with 20 columns a cell, and one
+// for face nodes.  An entry is a combination of the six products of the
+// gradients (p3_row_v, p3_row_e, p3_row_f, generated from exact integrals).
+// Bound by latency at 10 (V), 14 (E) and 16 (F) warps per SM: the FP64 pipe is
+// busy 12 % of the time, half of the instructions are integer ones (slots, the
+// stores of rows of 20 to 175 entries).  P3 n=36: 0.34 ms against 0.63 ms for
+// the warp-coalesced scatter (0.38 ms with one warp for a vertex group).
+// ---------------------------------------------------------------------------
+template <int COEF>
+__device__ __forceinline__ double cell_k(const WalkArgs& a, int c) {
+  if constexpr (COEF == FE_COEFF_DG0) return __ldg(a.coef + c);
+  else return a.coef_const;
+}
+
+// Vertex rows: two warps take the columns of each part (the nodes of vertices
+// and of the edges at a, and the others: never the same slot of a row), as the
+// segments of 175 slots leave room for few groups.
+template <int COEF, int PARTS>
+__global__ void __launch_bounds__(64 * PARTS) k_rows_v3(const WalkArgs a) {
+  extern __shared__ double smem[];
+  let_next_start();
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 6;
+  const bool outer = (threadIdx.x >> 5) & 1;
+  const int64_t g = blockIdx.x;
+  double* acc = smem + part * (32 * a.stride);
+  double* seg = acc + lane * a.stride;
+  const int4 own = __ldg(a.own + g * 32 + lane);
+  int s0 = __ldg(a.steps + g);
+  const int ns = (__ldg(a.steps + g + 1) - s0) / PARTS;
+  s0 += part * ns;
+  const uint4* rec = a.rec + (int64_t)s0 * 32 + lane;
+  const uint4* rec2 = a.rec2 + (int64_t)s0 * 32 + lane;
+  const int32_t* cell = a.cell + (int64_t)s0 * 32 + lane;
+  const uint4 none = make_uint4(kStripLoad, 0u, 0u, 0u), zero4 = make_uint4(0u, 0u, 0u, 0u);
+  // records two steps ahead, coordinates and coefficient one
+  uint4 w1 = ns > 0 ? __ldg(rec) : none, w2 = ns > 1 ? __ldg(rec + 32) : none;
+  uint4 u1 = ns > 0 ? __ldg(rec2) : zero4, u2 = ns > 1 ? __ldg(rec2 + 32) : zero4;
+  int c1 = COEF == FE_COEFF_DG0 && ns > 0 ? __ldg(cell) : 0, c2 = COEF == FE_COEFF_DG0 && ns > 1 ? __ldg(cell + 32) : 0;
+  const RowAt at = row_at(a, own.x);
+  V3 xa{0.0, 0.0, 0.0}, xr = load_x(a.x4, (int)(w1.x & kStripVertex)), ep{0.0, 0.0, 0.0}, eq{0.0, 0.0, 0.0};
+  double kn = cell_k<COEF>(a, c1);
+  if (own.y >= 0) xa = load_x(a.x4, own.y);
+  for (int s = outer ? 1 : 0; s < a.stride; s += 2) seg[s] = 0.0;
+  __syncthreads();
+  double diag = 0.0;
+  for (int s = 0; s < ns; ++s) {
+    const uint4 w = w1, u = u1;
+    w1 = w2;
+    u1 = u2;
+    c1 = c2;
+    w2 = s + 2 < ns ? __ldg(rec + (s + 2) * 32) : none;
+    u2 = s + 2 < ns ? __ldg(rec2 + (s + 2) * 32) : zero4;
+    if (COEF == FE_COEFF_DG0 && s + 2 < ns) c2 = __ldg(cell + (s + 2) * 32);
+    const V3 er = xr - xa;
+    const double k = kn;
+    xr = load_x(a.x4, (int)(w1.x & kStripVertex));
+    kn = cell_k<COEF>(a, c1);
+    if (!(w.x & kStripLoad)) {
+      const V3 gp = cross(eq, er), gq = cross(er, ep), gr = cross(ep, eq);
+      const V3 ga = neg_sum(gp, gq, gr);
+      const double f = k / fabs(dot(ep, gp));
+      const double gg[6] = {f * dot(ga, gp), f * dot(ga, gq), f * dot(ga, gr), 0.0, 0.0, 0.0};
+      const uint32_t word[6] = {w.y, w.z, w.w, u.x, u.y, 0u};
+      auto slot = [&](int j) { return (word[(j - 1) >> 2] >> (8 * ((j - 1) & 3))) & 0xffu; };
+      // a cell's columns differ: reads before writes
+      if (!outer) {
+        double v[10], o[10];
+        p3_row_v(gg, [&](int j, double x) {
+          if (j < 10) v[j] = x;
+        });
+        diag += v[0];
+#pragma unroll
+        for (int j = 1; j < 10; ++j) o[j] = seg[slot(j)];
+#pragma unroll
+        for (int j = 1; j < 10; ++j) seg[slot(j)] = o[j] + v[j];
+      } else {
+        double v[10], o[10];
+        p3_row_v(gg, [&](int j, double x) {
+          if (j >= 10) v[j - 10] = x;
+        });
+#pragma unroll
+        for (int j = 10; j < 20; ++j) o[j - 10] = seg[slot(j)];
+#pragma unroll
+        for (int j = 10; j < 20; ++j) seg[slot(j)] = o[j - 10] + v[j - 10];
+      }
+    }
+    if (!(w.x & kStripKeep)) ep = eq;
+    eq = er;
+  }
+  // (the row's own column: added by the inner warp alone)
+  if (own.y >= 0 && !outer) seg[own.w & 0xff] += diag;
+  __syncthreads();
+  if constexpr (PARTS > 1) {
+    for (int t = threadIdx.x; t < 32 * a.stride; t += 64 * PARTS) {
+      double v = smem[t];
+#pragma unroll
+      for (int q = 1; q < PARTS; ++q) v += smem[q * (32 * a.stride) + t];
+      smem[t] = v;
+    }
+    __syncthreads();
+  }
+  constexpr int kRows = 16 / PARTS;
+  store_rows(a, smem, at, own.w & 0xff, lane, (threadIdx.x >> 5) * kRows, kRows);
+}
+
+template <int COEF>
+__global__ void __launch_bounds__(32, kMinE3) k_rows_e3(const WalkArgs a) {
+  extern __shared__ double smem[];
+  let_next_start();
+  const int lane = threadIdx.x;
+  const int64_t g = blockIdx.x;
+  double* seg = smem + lane * a.stride;
+  const int4 own = __ldg(a.own + g * 32 + lane);
+  const int s0 = __ldg(a.steps + g), ns = __ldg(a.steps + g + 1) - s0;
+  const uint4 none = make_uint4(kAll, kAll, 0u, 0u);
+  const uint4* rec = a.rec + (int64_t)s0 * 32 + lane;
+  const uint4* rec2 = a.rec2 + (int64_t)s0 * 32 + lane;
+  const int32_t* cell = a.cell + (int64_t)s0 * 32 + lane;
+  uint4 w1 = ns > 0 ? __ldg(rec) : none, w2 = ns > 1 ? __ldg(rec + 32) : none;
+  int c1 = COEF == FE_COEFF_DG0 && ns > 0 ? __ldg(cell) : 0, c2 = COEF == FE_COEFF_DG0 && ns > 1 ? __ldg(cell + 32) : 0;
+  const RowAt at = row_at(a, own.x);
+  V3 xa{0.0, 0.0, 0.0}, e1{0.0, 0.0, 0.0}, ec{0.0, 0.0, 0.0}, xd{0.0, 0.0, 0.0};
+  double kn = cell_k<COEF>(a, c1);
+  if (own.y >= 0) {
+    xa = load_x(a.x4, own.y);
+    e1 = load_x(a.x4, own.z) - xa;
+  }
+  if (w1.y != kAll) xd = load_x(a.x4, (int)w1.y);
+  if (a.gaps)
+    for (int s = 0; s < a.stride; ++s) seg[s] = 0.0;
+  uint4 u1 = ns > 0 ? __ldg(rec2) : make_uint4(0u, 0u, 0u, 0u);
+  double mine[4] = {0.0, 0.0, 0.0, 0.0};             // columns a, b and the edge's two nodes
+  double run[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // the columns of c so far
+  for (int s = 0; s < ns; ++s) {
+    const uint4 w = w1;
+    w1 = w2;
+    c1 = c2;
+    w2 = s + 2 < ns ? __ldg(rec + (s + 2) * 32) : none;
+    if (COEF == FE_COEFF_DG0 && s + 2 < ns) c2 = __ldg(cell + (s + 2) * 32);
+    if (w.y == kAll) continue;
+    const uint4 u = u1;
+    if (s + 1 < ns) u1 = __ldg(rec2 + (s + 1) * 32);
+    if (u.z & kFanBegin) {
+      ec = load_x(a.x4, (int)w.x) - xa;
+#pragma unroll
+      for (int q = 0; q < 6; ++q) run[q] = 0.0;
+    }
+    const V3 ed = xd - xa;
+    const double k = kn;
+    if (w1.y != kAll) xd = load_x(a.x4, (int)w1.y);
+    kn = cell_k<COEF>(a, c1);
+    const V3 gb = cross(ec, ed), gc = cross(ed, e1), gd = cross(e1, ec);
+    const V3 ga = neg_sum(gb, gc, gd);
+    const double f = k / fabs(dot(e1, gb));
+    const double gg[6] = {f * dot(ga, gb), f * dot(ga, gc), f * dot(ga, gd), f * dot(gb, gc), f * dot(gb, gd), 0.0};
+    double v[20];
+    p3_row_e(gg, [&](int j, double x) { v[j] = x; });
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mine[q] += v[q];
+    const uint32_t cs[6] = {w.z & 0xffu, (w.z >> 8) & 0xffu, (w.z >> 16) & 0xffu,
+                            w.z >> 24,   w.w & 0xffu,        (w.w >> 8) & 0xffu};
+#pragma unroll
+    for (int q = 0; q < 6; ++q) seg[cs[q]] = run[q] + v[4 + q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) seg[(u.y >> (8 * q)) & 0xffu] = v[16 + q];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) run[q] = v[10 + q];
+    if (u.z & kFanEnd) {
+      const uint32_t ds[6] = {(w.w >> 16) & 0xffu, w.w >> 24,          u.x & 0xffu,
+                              (u.x >> 8) & 0xffu,  (u.x >> 16) & 0xffu, u.x >> 24};
+      if (u.z & kFanClosed) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) run[q] += seg[ds[q]];
+      }
+#pragma unroll
+      for (int q = 0; q < 6; ++q) seg[ds[q]] = run[q];
+    }
+    ec = ed;
+  }
+  if (own.y >= 0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) seg[((uint32_t)own.w >> (8 * q)) & 0xffu] = mine[q];
+  }
+  store_rows(a, smem, at, (own.w >> 16) & 0xff, lane, 0, 32);
+  end_after_previous();
+}
+
+// Face rows: one or two cells, which share the face's ten nodes only.
+template <int COEF>
+__global__ void __launch_bounds__(32, kMinF3) k_rows_f3(const WalkArgs a) {
+  extern __shared__ double smem[];
+  let_next_start();
+  const int lane = threadIdx.x;
+  const int64_t g = blockIdx.x;
+  double* seg = smem + lane * a.stride;
+  const int4 own = __ldg(a.own + g * 32 + lane);
+  const int s0 = __ldg(a.steps + g), ns = __ldg(a.steps + g + 1) - s0;
+  const uint4 none = make_uint4(kAll, 0u, 0u, 0u);
+  const uint4* rec = a.rec + (int64_t)s0 * 32 + lane;
+  const int32_t* cell = a.cell + (int64_t)s0 * 32 + lane;
+  uint4 w1 = ns > 0 ? __ldg(rec) : none;
+  int c1 = COEF == FE_COEFF_DG0 && ns > 0 ? __ldg(cell) : 0;
+  const RowAt at = row_at(a, own.x);
+  const int4 slots = __ldg(a.own2 + g * 32 + lane);
+  V3 xa{0.0, 0.0, 0.0}, e1{0.0, 0.0, 0.0}, e2{0.0, 0.0, 0.0};
+  if (own.y >= 0) {
+    xa = load_x(a.x4, own.y);
+    e1 = load_x(a.x4, own.z) - xa;
+    e2 = load_x(a.x4, own.w) - xa;
+  }
+  const V3 gd = cross(e1, e2);
+  if (a.gaps)
+    for (int s = 0; s < a.stride; ++s) seg[s] = 0.0;
+  double mine[10];
+#pragma unroll
+  for (int q = 0; q < 10; ++q) mine[q] = 0.0;
+  for (int s = 0; s < ns; ++s) {
+    const uint4 w = w1;
+    const int c = c1;
+    if (s + 1 < ns) {
+      w1 = __ldg(rec + (s + 1) * 32);
+      if (COEF == FE_COEFF_DG0) c1 = __ldg(cell + (s + 1) * 32);
+    }
+    if (w.x == kAll) continue;
+    const V3 e3 = load_x(a.x4, (int)w.x) - xa;
+    const double k = cell_k<COEF>(a, c);
+    const V3 gb = cross(e2, e3), gc = cross(e3, e1);
+    const V3 ga = neg_sum(gb, gc, gd);
+    const double f = k / fabs(dot(e1, gb));
+    const double gg[6] = {f * dot(ga, gb), f * dot(ga, gc), f * dot(ga, gd),
+                          f * dot(gb, gc), f * dot(gb, gd), f * dot(gc, gd)};
+    const uint32_t word[3] = {w.y, w.z, w.w};
+    p3_row_f(gg, [&](int j, double x) {
+      if (j < 10) mine[j] += x;
+      else seg[(word[(j - 10) >> 2] >> (8 * ((j - 10) & 3))) & 0xffu] = x;
+    });
+  }
+  if (own.y >= 0) {
+    const uint32_t word[3] = {(uint32_t)slots.x, (uint32_t)slots.y, (uint32_t)slots.z};
+#pragma unroll
+    for (int q = 0; q < 10; ++q) seg[(word[q >> 2] >> (8 * (q & 3))) & 0xffu] = mine[q];
+  }
+  store_rows(a, smem, at, (slots.z >> 8) & 0xff, lane, 0, 32);
+  end_after_previous();
+}
+
 unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 int odd_at_least(int n) { return n | 1; }
@@ -1036,8 +1357,22 @@ int degree_of(int kind) {
   switch (kind) {
     case FE_FORM_P1_STIFFNESS: return 1;
     case FE_FORM_P2_STIFFNESS: return 2;
+    case FE_FORM_P3_STIFFNESS: return 3;
     default: return 0;
   }
+}
+
+template <int COEF>
+void raise_p3_of() {
+  raise_smem(k_rows_v3<COEF, 1>);
+  raise_smem(k_rows_v3<COEF, 2>);
+  raise_smem(k_rows_v3<COEF, 4>);
+  raise_smem(k_rows_e3<COEF>);
+  raise_smem(k_rows_f3<COEF>);
+}
+void raise_p3() {
+  raise_p3_of<FE_COEFF_CONSTANT>();
+  raise_p3_of<FE_COEFF_DG0>();
 }
 
 void exclusive_scan(int32_t* v, int64_t n, cudaStream_t s) {
@@ -1081,6 +1416,11 @@ void build_part(const PlanArgs& a, PartArgs p, fe_form_s::RowsPlan::Part& part, 
   part.ngroups = p.ngroups;
   part.parts = p.parts;
   part.own.alloc((size_t)p.ngroups * 32);
+  if (p.kind == KIND_F) {
+    part.own2.alloc((size_t)p.ngroups * 32);
+    FE_CUDA(cudaMemsetAsync(part.own2.p, 0, part.own2.bytes(), s));
+    p.own2 = part.own2.p;
+  }
   part.steps.alloc((size_t)p.ngroups + 1);
   DevBuf<unsigned> gaps(1);
   FE_CUDA(cudaMemsetAsync(gaps.p, 0, sizeof(unsigned), s));
@@ -1101,8 +1441,10 @@ void build_part(const PlanArgs& a, PartArgs p, fe_form_s::RowsPlan::Part& part, 
   const size_t nrec = (size_t)total * 32;
   if (a.deg == 1) part.rec1.alloc(std::max<size_t>(1, nrec));
   else part.rec.alloc(std::max<size_t>(1, nrec));
+  if (a.deg == 3 && p.kind != KIND_F) part.rec2.alloc(std::max<size_t>(1, nrec));
   part.cell.alloc(std::max<size_t>(1, nrec));
   p.rec = part.rec.p;
+  p.rec2 = part.rec2.p;
   p.rec1 = part.rec1.p;
   p.cell = part.cell.p;
   k_rows_records<<<blocks_for(p.ngroups * 32, 128), 128, 0, s>>>(a, p);
@@ -1133,12 +1475,14 @@ void reset_rows_plan(fe_form_s& f) { f.rows_plan.reset(); }
 // Small meshes keep the scatter: a call's time is its launches there and the
 // plan would not pay.  On B200, us per call, walk / best scatter: P1 n=20
 // (48,000 cells) 8.4 / 9.1, n=32 (196,608) 13.7 / 16.7, n=45 28 / 35; P2 n=16
-// (24,576) 16 / 18, n=20 25 / 25, n=28 (131,712) 42 / 64.
+// (24,576) 16 / 18, n=20 25 / 25, n=28 (131,712) 42 / 64; P3 n=3 27 / 59,
+// n=12 29 / 65, n=20 86 / 105.
 bool rows_default(const fe_form_s& f) {
   const int64_t cells = f.mesh ? f.mesh->num_cells : 0;
   switch (degree_of(f.kind)) {
     case 1: return cells >= 98304;
     case 2: return cells >= 65536;
+    case 3: return true;
     default: return false;
   }
 }
@@ -1226,22 +1570,24 @@ void build_rows_plan(fe_form_s& f, cudaStream_t s) {
     FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaStreamSynchronize(s));  // the temporaries are freed on return
     if (bad) return;
-    // the rows of a kind: a longer bound than needed for the others is fine
-    // for P1 and P2 edge rows are the shorter ones
-    P->part[KIND_V].stride = odd_at_least(longest);
-    int longest_e = 0;
-    if (hk[KIND_E]) {
-      std::vector<int32_t> he((size_t)hk[KIND_E]);
-      FE_CUDA(cudaMemcpy(he.data(), row_sorted.p + hk[KIND_V], he.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
-      for (int32_t r : he) longest_e = std::max(longest_e, f.sp->host_row_ptr[r + 1] - f.sp->host_row_ptr[r]);
+    // segments as long as the longest row of the kind
+    std::vector<int32_t> order((size_t)nR);
+    FE_CUDA(cudaMemcpy(order.data(), row_sorted.p, order.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    int64_t at = 0;
+    for (int kind = 0; kind < 3; ++kind) {
+      int len = 0;
+      for (const int64_t end = at + hk[kind]; at < end; ++at)
+        len = std::max(len, f.sp->host_row_ptr[order[at] + 1] - f.sp->host_row_ptr[order[at]]);
+      P->part[kind].stride = odd_at_least(len);
     }
-    P->part[KIND_E].stride = odd_at_least(longest_e);
     // at least four warps per SM, or the scatter is the better one
-    if (segment_bytes(P->part[KIND_V].stride) + kSmemCta > kSmemSm / 4 ||
-        segment_bytes(P->part[KIND_E].stride) + kSmemCta > kSmemSm / 4)
-      return;
+    for (auto& part : P->part) {
+      if (segment_bytes(part.stride) + kSmemCta > kSmemSm / 4) return;
+      while (part.parts > 1 && part.parts * segment_bytes(part.stride) + kSmemCta > kSmemSm) part.parts /= 2;
+    }
     if (deg == 1) raise_all<1>();
-    else raise_all<2>();
+    else if (deg == 2) raise_all<2>();
+    else raise_p3();
     if (deg == 2) {
       raise_smem(k_rows_e2<FE_COEFF_CONSTANT>);
       raise_smem(k_rows_e2<FE_COEFF_DG0>);
@@ -1260,7 +1606,7 @@ bool rows_supported(fe_form_s& f, const fe_bc_s* bc0, const fe_bc_s* bc1, cudaSt
   if (!f.rows_plan || f.precision != FE_PREC_FP64 || bc0 != bc1) return false;
   const Coefficient& k = f.coeff[0];
   if (k.kind == FE_COEFF_P1) {
-    if (!k.map || !vertex_numbered(f, *k.map, s)) return false;
+    if (f.kind == FE_FORM_P3_STIFFNESS || !k.map || !vertex_numbered(f, *k.map, s)) return false;
   } else if (k.kind != FE_COEFF_DG0 && k.kind != FE_COEFF_CONSTANT && k.kind >= 0) {
     return false;
   }
@@ -1293,6 +1639,8 @@ void launch_parts(const fe_form_s& f, WalkArgs a, cudaStream_t s) {
     a.own = p.own.p;
     a.steps = p.steps.p;
     a.rec = p.rec.p;
+    a.rec2 = p.rec2.p;
+    a.own2 = p.own2.p;
     a.rec1 = p.rec1.p;
     a.cell = p.cell.p;
     a.stride = p.stride;
@@ -1312,6 +1660,45 @@ void launch_parts(const fe_form_s& f, WalkArgs a, cudaStream_t s) {
   if (DEG == 2 && pe.ngroups) {
     set(pe);
     launch_beside(k_rows_e2<COEF>, (unsigned)pe.ngroups, segment_bytes(pe.stride), pv.ngroups > 0, a, s);
+  }
+}
+
+template <int COEF>
+void launch_p3(const fe_form_s& f, WalkArgs a, cudaStream_t s) {
+  const fe_form_s::RowsPlan& P = *f.rows_plan;
+  auto set = [&](const fe_form_s::RowsPlan::Part& p) {
+    a.ngroups = p.ngroups;
+    a.own = p.own.p;
+    a.own2 = p.own2.p;
+    a.steps = p.steps.p;
+    a.rec = p.rec.p;
+    a.rec2 = p.rec2.p;
+    a.cell = p.cell.p;
+    a.stride = p.stride;
+    a.gaps = p.gaps ? 1 : 0;
+    return (unsigned)p.ngroups;
+  };
+  bool beside = false;
+  const auto& pv = P.part[KIND_V];
+  if (pv.ngroups) {
+    const unsigned grid = set(pv);
+    const size_t seg = segment_bytes(pv.stride);
+    if (pv.parts == 4) k_rows_v3<COEF, 4><<<grid, 256, 4 * seg, s>>>(a);
+    else if (pv.parts == 2) k_rows_v3<COEF, 2><<<grid, 128, 2 * seg, s>>>(a);
+    else k_rows_v3<COEF, 1><<<grid, 64, seg, s>>>(a);
+    FE_CUDA(cudaGetLastError());
+    beside = true;
+  }
+  const auto& pe = P.part[KIND_E];
+  if (pe.ngroups) {
+    const unsigned grid = set(pe);
+    launch_beside(k_rows_e3<COEF>, grid, segment_bytes(pe.stride), beside, a, s);
+    beside = true;
+  }
+  const auto& pf = P.part[KIND_F];
+  if (pf.ngroups) {
+    const unsigned grid = set(pf);
+    launch_beside(k_rows_f3<COEF>, grid, segment_bytes(pf.stride), beside, a, s);
   }
 }
 }  // namespace
@@ -1350,7 +1737,10 @@ void assemble_matrix_rows(fe_form_s& f, double* values, const fe_bc_s* bc, doubl
     set_diag = !owned || !zero;
   }
   const int kind = k.kind < 0 ? FE_COEFF_CONSTANT : k.kind;
-  if (f.kind == FE_FORM_P1_STIFFNESS) {
+  if (f.kind == FE_FORM_P3_STIFFNESS) {
+    if (kind == FE_COEFF_DG0) launch_p3<FE_COEFF_DG0>(f, a, s);
+    else launch_p3<FE_COEFF_CONSTANT>(f, a, s);
+  } else if (f.kind == FE_FORM_P1_STIFFNESS) {
     if (kind == FE_COEFF_P1) launch_parts<1, FE_COEFF_P1>(f, a, s);
     else if (kind == FE_COEFF_DG0) launch_parts<1, FE_COEFF_DG0>(f, a, s);
     else launch_parts<1, FE_COEFF_CONSTANT>(f, a, s);

@@ -379,6 +379,7 @@ def gen() -> str:
         w("    " + ", ".join(vals[k:k + 6]) + ",\n")
     w("};\n\n")
     w(mass_tables())
+    w(p3_row_tables())
     w(facet_tables())
     w("}  // namespace fe\n")
     return "".join(out)
@@ -422,6 +423,109 @@ def mass_tables() -> str:
             exprs[(i, j)] = sum_expr("cq", terms, 2)
         w(plain_symmetric_body(exprs))
         w("}\n\n")
+    return "".join(out)
+
+
+def p3_row_tables() -> str:
+    """Rows of the P3 stiffness tensor in a row's own vertex order (fe_rows.cu):
+    the node is vertex a, the node of edge ab near a, or the node of face abc.
+    With g_x the gradients of the barycentric coordinates, an entry is
+    sum_xy c_xy g_x.g_y, c_xy = int d_x phi_i d_y phi_j over the barycentric
+    derivatives; g_x.g_x = -sum_{y != x} g_x.g_y leaves the six products x < y."""
+    lam = [tuple(1 if q == v else 0 for q in range(4)) for v in range(4)]
+
+    def mul(p, q):
+        r = {}
+        for k1, v1 in p.items():
+            for k2, v2 in q.items():
+                k = tuple(x + y for x, y in zip(k1, k2))
+                r[k] = r.get(k, 0) + v1 * v2
+        return r
+
+    def lin(v, c, d):  # c * lambda_v + d
+        r = {lam[v]: Fraction(c)}
+        if d:
+            r[(0, 0, 0, 0)] = Fraction(d)
+        return r
+
+    def scale(p, c):
+        return {k: v * c for k, v in p.items()}
+
+    def diff(p, x):
+        r = {}
+        for k, v in p.items():
+            if k[x]:
+                kk = list(k)
+                kk[x] -= 1
+                r[tuple(kk)] = r.get(tuple(kk), 0) + v * k[x]
+        return r
+
+    def integral(p):  # over the tetrahedron, divided by |det J|
+        t = Fraction(0)
+        for k, v in p.items():
+            t += v * Fraction(factorial(k[0]) * factorial(k[1]) * factorial(k[2]) * factorial(k[3]),
+                              factorial(sum(k) + 3))
+        return t
+
+    def vertex(v):
+        return scale(mul(lin(v, 1, 0), mul(lin(v, 3, -1), lin(v, 3, -2))), Fraction(1, 2))
+
+    def edge(near, far):
+        return scale(mul(mul(lin(near, 1, 0), lin(far, 1, 0)), lin(near, 3, -1)), Fraction(9, 2))
+
+    def face(f):
+        o = [v for v in range(4) if v != f]
+        return scale(mul(mul(lin(o[0], 1, 0), lin(o[1], 1, 0)), lin(o[2], 1, 0)), Fraction(27))
+
+    a, b, c, d = range(4)
+    cols = {
+        "v": [vertex(a), vertex(b), vertex(c), vertex(d), edge(a, b), edge(b, a), edge(a, c), edge(c, a), edge(a, d),
+              edge(d, a), edge(b, c), edge(c, b), edge(b, d), edge(d, b), edge(c, d), edge(d, c), face(d), face(c),
+              face(b), face(a)],
+        "e": [vertex(a), vertex(b), edge(a, b), edge(b, a), vertex(c), edge(a, c), edge(c, a), edge(b, c), edge(c, b),
+              face(d), vertex(d), edge(a, d), edge(d, a), edge(b, d), edge(d, b), face(c), edge(c, d), edge(d, c),
+              face(b), face(a)],
+        "f": [vertex(a), vertex(b), vertex(c), edge(a, b), edge(b, a), edge(a, c), edge(c, a), edge(b, c), edge(c, b),
+              face(d), vertex(d), edge(a, d), edge(d, a), edge(b, d), edge(d, b), edge(c, d), edge(d, c), face(c),
+              face(b), face(a)],
+    }
+    row = {"v": vertex(a), "e": edge(a, b), "f": face(d)}
+    what = {"v": "vertex a", "e": "the node of edge ab near a", "f": "the node of face abc"}
+    order = {
+        "v": "a, b, c, d, ab ba ac ca ad da bc cb bd db cd dc (xy: on edge xy near x), abc abd acd bcd",
+        "e": "a, b, ab, ba, c, ac ca bc cb, abc, d, ad da bd db, abd, cd dc, acd, bcd",
+        "f": "a, b, c, ab ba ac ca bc cb, abc, d, ad da bd db cd dc, abd, acd, bcd",
+    }
+    pairs = [(a, b), (a, c), (a, d), (b, c), (b, d), (c, d)]
+    out = []
+    for kind in ("v", "e", "f"):
+        out.append(f"// P3 stiffness row of {what[kind]}: g[q] = k |det J| times the products of the gradients\n"
+                   f"// ab, ac, ad, bc, bd, cd; emit(column, value), columns {order[kind]}.\n")
+        body, table = [], []
+        for j, q in enumerate(cols[kind]):
+            cxy = [[integral(mul(diff(row[kind], x), diff(q, y))) for y in range(4)] for x in range(4)]
+            terms = []
+            for t, (x, y) in enumerate(pairs):
+                v = cxy[x][y] + cxy[y][x] - cxy[x][x] - cxy[y][y]
+                if v != 0:
+                    terms.append((t, v))
+            parts = []
+            for k in range(min(2, len(terms))):
+                e = ""
+                for t, v in terms[k::2]:
+                    if v not in table:
+                        table.append(v)
+                    ref = f"kP3Row{kind.upper()}[{table.index(v)}]"
+                    e = f"fma(g[{t}], {ref}, {e})" if e else f"g[{t}] * {ref}"
+                parts.append(e)
+            body.append(f"  emit({j}, {' + '.join(parts) if parts else '0.0'});\n")
+        out.append(f"__constant__ double kP3Row{kind.upper()}[{len(table)}] = {{\n")
+        for k in range(0, len(table), 6):
+            out.append("    " + ", ".join(lit(v) for v in table[k:k + 6]) + ",\n")
+        out.append("};\ntemplate <typename Emit>\n")
+        out.append(f"__device__ __forceinline__ void p3_row_{kind}(const double* g, Emit&& emit) {{\n")
+        out += body
+        out.append("}\n\n")
     return "".join(out)
 
 

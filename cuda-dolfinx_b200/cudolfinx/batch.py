@@ -27,10 +27,10 @@ CANDIDATES = {
     "P1_STIFFNESS": ("atomic", "block", "tile", "row-walk"),
     "P2_STIFFNESS": ("atomic", "block", "grouped", "coalesced", "row-walk"),
     "VP2_ELASTICITY": ("coalesced", "atomic", "atomic-full"),
-    "P3_STIFFNESS": ("coalesced", "atomic"),  # coalesced: FP64 element tensors only (skipped for FP32)
+    "P3_STIFFNESS": ("coalesced", "atomic", "row-walk"),  # coalesced, row-walk: FP64 element tensors only (skipped for FP32)
 }
 # the row walk is timed from the sizes on where it is the engine's default
-ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536}
+ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536, "P3_STIFFNESS": 0}
 # launch shapes of the atomic scatter timed per form kind: (cells per CTA,
 # byte maps staged in shared memory)
 LAUNCHES = {

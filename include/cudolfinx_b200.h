@@ -131,10 +131,10 @@ enum fe_precision {
                                      lanes on one cell's CSR row, so an instruction's reductions
                                      share L2 sectors); FE_ASM_ATOMIC keeps one thread's reductions
                                      per cell                                                       */
-#define FE_ASM_ROW_WALK 1024u     /* FP64 P1 / P2 stiffness: one thread per CSR row walks the cells around
+#define FE_ASM_ROW_WALK 1024u     /* FP64 P1 / P2 / P3 stiffness: one thread per CSR row walks the cells around
                                      the row's node and stores the row once, without reductions or a
                                      zero pass (reproducible); the default from 98,304 (P1) and 65,536
-                                     (P2) cells on, below which the call asks for it by this flag; needs
+                                     (P2) cells on and for P3, below which the call asks for it by this flag; needs
                                      one space and one set of BCs for rows and columns               */
 
 /* ---- errors / context --------------------------------------------------- */

@@ -1,4 +1,4 @@
-"""The row walk (variant "row-walk", the default of large FP64 P1 / P2 matrices) against
+"""The row walk (variant "row-walk", the default of large FP64 P1 / P2 / P3 matrices) against
 the thread-per-cell scatter into both triangles (variant "atomic-full").
 
 The element matrices are positive semi-definite, so the sum of an entry's
@@ -13,7 +13,7 @@ from conftest import ensure_library
 
 pytestmark = pytest.mark.gpu
 
-SPACE = {"p1": ("P", 1), "p2": ("P", 2)}
+SPACE = {"p1": ("P", 1), "p2": ("P", 2), "p3": ("P", 3)}
 
 
 def _mesh(n, order, seed=0, cells=None):
@@ -85,9 +85,12 @@ def _compare(V, a, bcs, diagonal=1.0, variant="row-walk"):
 
 @pytest.mark.parametrize("order", ["natural", "permuted"])
 @pytest.mark.parametrize("coef", ["const", "dg0", "p1"])
-@pytest.mark.parametrize("kind,n", [("p1", 1), ("p1", 3), ("p1", 10), ("p2", 1), ("p2", 2), ("p2", 7), ("p1", 33), ("p2", 23)])
+@pytest.mark.parametrize("kind,n", [("p1", 1), ("p1", 3), ("p1", 10), ("p2", 1), ("p2", 2), ("p2", 7), ("p1", 33), ("p2", 23),
+                                    ("p3", 1), ("p3", 2), ("p3", 5)])
 def test_walk_matches_scatter(kind, n, coef, order):
     ensure_library()
+    if kind == "p3" and coef == "p1":
+        pytest.skip("P3 stiffness takes a constant or cellwise coefficient")
     from cudolfinx import fem
 
     mesh = _mesh(n, order, seed=n)
@@ -97,7 +100,7 @@ def test_walk_matches_scatter(kind, n, coef, order):
 
 
 @pytest.mark.parametrize("cells", [[0], [0, 3], [0, 1, 3, 4], [5, 4, 2, 0], [0, 1, 2, 3, 4]])
-@pytest.mark.parametrize("kind", ["p1", "p2"])
+@pytest.mark.parametrize("kind", ["p1", "p2", "p3"])
 def test_open_and_separate_fans(kind, cells):
     """Some of the six cells around the cube's diagonal: one cell, cells that
     share only an edge (two fans), open fans; nodes of no cell."""
@@ -105,14 +108,14 @@ def test_open_and_separate_fans(kind, cells):
     from cudolfinx import fem
 
     mesh = _mesh(1, "natural", cells=cells)
-    V, a = _form(kind, "p1", mesh)
+    V, a = _form(kind, "dg0" if kind == "p3" else "p1", mesh)
     _compare(V, a, [fem.dirichletbc(0.0, np.array([0, V.num_dofs - 1]), V)])
 
 
-@pytest.mark.parametrize("kind", ["p1", "p2"])
+@pytest.mark.parametrize("kind", ["p1", "p2", "p3"])
 def test_overlapping_cells(kind):
     """Cells listed twice: a vertex row adds them all; a walk around an edge
-    writes each slot once, so P2 refuses them and "auto" takes the scatter."""
+    writes each slot once, so P2 and P3 refuse them and "auto" takes the scatter."""
     ensure_library()
     import cudolfinx as cx
     from cudolfinx import fem
@@ -121,12 +124,12 @@ def test_overlapping_cells(kind):
     V, a = _form(kind, "dg0", mesh)
     _compare(V, a, [fem.dirichletbc(0.0, fem.locate_boundary_dofs(V), V)],
              variant="row-walk" if kind == "p1" else "auto")
-    if kind == "p2":
+    if kind != "p1":
         with pytest.raises(RuntimeError, match="row walk"):
             cx.CUDAAssembler().assemble_matrix(a, variant="row-walk")
 
 
-@pytest.mark.parametrize("kind", ["p1", "p2"])
+@pytest.mark.parametrize("kind", ["p1", "p2", "p3"])
 def test_pattern_with_more_slots(kind):
     """A pattern with couplings the form does not have: their slots are zero."""
     ensure_library()
