@@ -745,6 +745,7 @@ int fe_form_bind_sparsity(fe_form f, fe_sparsity s, void* stream) {
       launch_build_slotmap(*f, st);
       check_device_errors(f->ctx, st, FE_ERR_PATTERN);
       if (rows_default(*f)) build_rows_plan(*f, st);
+      if (vp2_rows_default(*f)) build_nodes_plan(*f, st);
     } catch (...) {
       f->sp = nullptr;  // the byte map is incomplete: the form stays unbound
       throw;
@@ -971,9 +972,10 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
       if (bc0) launch_set_diagonal(*a->sp, *bc0, diagonal, values, st);
       return;
     }
-    // default: the block variant for P1 meshes above ~1M cells (measured faster
-    // on B200 at 12.6M cells: 0.54 vs 0.73 ms), the FP64-atomic scatter otherwise
-    // (for P2 stiffness with warp-coalesced reductions, below)
+    // default: the row walk wherever the form has its plan; else the block
+    // variant for P1 meshes above ~1M cells (measured faster on B200 at 12.6M
+    // cells: 0.54 vs 0.73 ms) and the FP64-atomic scatter otherwise (for P2
+    // stiffness and vector P2 with warp-coalesced reductions, below)
     const bool auto_block = !(flags & FE_ASM_ATOMIC) && !view && a->kind == FE_FORM_P1_STIFFNESS &&
                             a->mesh->num_cells >= (int64_t(1) << 20);
     const bool want_block = (flags & FE_ASM_BLOCK) || auto_block;
@@ -982,13 +984,20 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
     // bound) and no other variant is asked for
     if (flags & FE_ASM_ROW_WALK) {
       if (!a->rows_plan && !view) build_rows_plan(*a, st);
-      FE_REQUIRE(!view && rows_supported(*a, bc0, bc1, st),
-                 "the row walk supports FP64 P1/P2/P3 stiffness with one space and one set of BCs, on conforming cells");
+      if (!a->nodes_plan && !view) build_nodes_plan(*a, st);
+      FE_REQUIRE(!view && (rows_supported(*a, bc0, bc1, st) || vp2_rows_supported(*a, bc0, bc1, st)),
+                 "the row walk supports FP64 P1/P2/P3 stiffness and FP32 vector-P2 elasticity with one space and one "
+                 "set of BCs, on conforming cells");
     }
-    if (!(flags & (FE_ASM_ATOMIC | FE_ASM_FULL_SCATTER | FE_ASM_BLOCK | FE_ASM_COALESCED | FE_ASM_GROUPED)) && !view &&
-        rows_supported(*a, bc0, bc1, st)) {
-      assemble_matrix_rows(*a, values, bc0, diagonal, zero, st);
-      return;
+    if (!(flags & (FE_ASM_ATOMIC | FE_ASM_FULL_SCATTER | FE_ASM_BLOCK | FE_ASM_COALESCED | FE_ASM_GROUPED)) && !view) {
+      if (rows_supported(*a, bc0, bc1, st)) {
+        assemble_matrix_rows(*a, values, bc0, diagonal, zero, st);
+        return;
+      }
+      if (vp2_rows_supported(*a, bc0, bc1, st)) {
+        assemble_matrix_vp2_rows(*a, values, bc0, diagonal, zero, st);
+        return;
+      }
     }
     if (want_block && block_supported(*a)) {
       assemble_matrix_block(*a, values, bc0, bc1, zero, diagonal, st);

@@ -28,6 +28,7 @@ void fe::reset_gather_plan(fe_form_s& f) {
   reset_tile_plan(f);
   reset_row_plan(f);
   reset_rows_plan(f);
+  reset_nodes_plan(f);
   reset_block_plan(f);
   reset_batch_plan(f);
 }

@@ -234,6 +234,9 @@ struct fe_form_s {
   // the walk does not apply
   struct RowsPlan;
   std::unique_ptr<RowsPlan> rows_plan;
+  // vector-P2 row walk (fe_rows_vp2.cu), likewise
+  struct NodesPlan;
+  std::unique_ptr<NodesPlan> nodes_plan;
 
   bool group_plan_failed = false;  // the mesh has no repeated group structure
   fe_form_s();
@@ -320,6 +323,20 @@ struct fe_form_s::RowsPlan {
   fe::DevBuf<double4> x4;             // vertex coordinates, 32 bytes apart
   uint64_t map_id = 0;                // P1 coefficient dofmap last compared with the mesh's vertices
   bool map_same = false;
+};
+
+struct fe_form_s::NodesPlan {
+  // nodes of one kind (vertices, edge nodes) in groups of three; record (step, node)
+  // of a group stands at (steps[group] + step) * 3 + node
+  struct Part {
+    int64_t ngroups = 0;
+    int stride = 0;                   // doubles of a node's segment in shared memory (even)
+    fe::DevBuf<int4> own;             // [groups*3] its first row (-1: none), where that begins, row length << 8
+                                      // and the slot of its own column, the group's last step + 1
+    fe::DevBuf<int32_t> steps;        // [groups+1] prefix sums of the groups' most cells
+    fe::DevBuf<uint4> rec;            // cell, local node, slot bytes
+  };
+  Part part[2];
 };
 
 struct fe_form_s::BlockPlan {
@@ -566,6 +583,13 @@ void reset_rows_plan(fe_form_s& f);
 bool rows_supported(fe_form_s& f, const fe_bc_s* bc0, const fe_bc_s* bc1, cudaStream_t s);
 void assemble_matrix_rows(fe_form_s& f, double* values, const fe_bc_s* bc, double diagonal, bool zero,
                           cudaStream_t s);
+// the same for vector-P2 elasticity (fe_rows_vp2.cu)
+bool vp2_rows_default(const fe_form_s& f);
+void build_nodes_plan(fe_form_s& f, cudaStream_t s);
+void reset_nodes_plan(fe_form_s& f);
+bool vp2_rows_supported(const fe_form_s& f, const fe_bc_s* bc0, const fe_bc_s* bc1, cudaStream_t s);
+void assemble_matrix_vp2_rows(fe_form_s& f, double* values, const fe_bc_s* bc, double diagonal, bool zero,
+                              cudaStream_t s);
 
 // row-gather assembly (fe_rowgather.cu) for P1 stiffness
 bool rowgather_supported(const fe_form_s& f);

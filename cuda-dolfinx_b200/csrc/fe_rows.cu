@@ -36,15 +36,13 @@
 
 #include "fe_element_code.cuh"
 #include "fe_internal.h"
+#include "fe_rows.cuh"
 
 namespace fe {
 namespace {
 
-constexpr unsigned kAll = 0xffffffffu;
 constexpr int kMaxStar = 128;           // cells of a vertex row
 constexpr int kStripTries = 64;         // beginnings tried for its walk
-constexpr size_t kSmemSm = 227 * 1024;  // shared memory one SM gives to its CTAs
-constexpr size_t kSmemCta = 1024;       // the part the system takes of each CTA's share
 
 // marks of an edge row's record: the first and the last cell of a fan around
 // the edge; a closed fan ends at the vertex it began with
@@ -647,34 +645,10 @@ __global__ void k_rows_same_map(const int32_t* __restrict__ m, const int32_t* __
   if (t < n && m[t] != g[t]) *differ = 1u;
 }
 
-// bit s of the mask: the column of slot s is a BC column
-__global__ void k_rows_bc_mask(const int32_t* __restrict__ col, int64_t nnz, const uint8_t* __restrict__ markers,
-                               uint32_t* __restrict__ mask) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const unsigned b = __ballot_sync(kAll, q < nnz && markers[col[q]] != 0);
-  if ((threadIdx.x & 31) == 0 && q < nnz) mask[q >> 5] = b;
-}
-// bit 0: a BC row; bit 1: a row with a BC column
-__global__ void k_rows_bc_flags(const int32_t* __restrict__ row_ptr, int64_t num_rows,
-                                const uint8_t* __restrict__ markers, const uint32_t* __restrict__ mask,
-                                uint8_t* __restrict__ flags) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= num_rows) return;
-  const int32_t lo = row_ptr[r], hi = row_ptr[r + 1];
-  uint32_t any = 0u;
-  for (int32_t w = lo >> 5; w <= (hi - 1) >> 5 && lo < hi; ++w) {
-    uint32_t m = mask[w];
-    if (w == lo >> 5) m &= kAll << (lo & 31);
-    if (w == (hi - 1) >> 5) m &= kAll >> (31 - ((hi - 1) & 31));
-    any |= m;
-  }
-  flags[r] = (uint8_t)((markers[r] ? 1 : 0) | (any ? 2 : 0));
-}
-
 // ---------------------------------------------------------------------------
 // assembly
 // ---------------------------------------------------------------------------
-struct WalkArgs {
+struct WalkArgs : RowOut {
   int64_t ngroups;
   const int4* __restrict__ own;
   const int32_t* __restrict__ steps;
@@ -684,16 +658,9 @@ struct WalkArgs {
   const uint2* __restrict__ rec1;
   const int32_t* __restrict__ cell;
   const double4* __restrict__ x4;
-  int stride;     // doubles between the segments of a warp's rows (odd)
   int gaps;       // some rows have slots that no cell adds to
   const double* __restrict__ coef;   // DG0: [cells]; P1: [vertices]
   double coef_const;
-  const int32_t* __restrict__ row_ptr;
-  const uint8_t* __restrict__ flags;  // BC flags of the rows, or null
-  const uint32_t* __restrict__ mask;  // bit s: the column of slot s is a BC column
-  double diagonal;   // stored on BC rows (with zero)
-  int zero;
-  double* __restrict__ values;
 };
 
 struct V3 {
@@ -714,100 +681,11 @@ __device__ __forceinline__ V3 load_x(const double4* __restrict__ x4, int v) {
   return {a.x, a.y, b};
 }
 
-// a lane's row in the value array, fetched before the walk
-struct RowAt {
-  int lo = 0, len = 0, fl = 0;
-};
-__device__ __forceinline__ RowAt row_at(const WalkArgs& a, int row) {
-  RowAt r;
-  if (row >= 0) {
-    r.lo = __ldg(a.row_ptr + row);
-    r.len = __ldg(a.row_ptr + row + 1) - r.lo;
-    if (a.flags) r.fl = __ldg(a.flags + row);
-  }
-  return r;
-}
-
-// The warp's 32 row segments (lane l's at acc + l * stride) to their rows.
-// First the segments of rows that a BC touches take their zeros (and a BC row
-// `diagonal` at its own slot), then all rows are stored, or added with zero == 0.
-// A warp takes the `count` rows from `first` on.
-__device__ __forceinline__ void store_rows(const WalkArgs& a, double* acc, const RowAt& at, int own_slot, int lane,
-                                           int first, int count) {
-  const unsigned mine = count == 32 ? kAll : ((1u << count) - 1u) << first;
-  __syncwarp();
-  // about every second warp has such rows, a few of them: four at a time, so
-  // that their mask words are fetched together
-  for (unsigned todo = __ballot_sync(kAll, at.fl != 0) & mine; todo;) {
-    int rr[4], rlo[4], rlen[4], rfl[4], rown[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      rr[q] = todo ? __ffs(todo) - 1 : 0;
-      rlo[q] = __shfl_sync(kAll, at.lo, rr[q]);
-      const int len = __shfl_sync(kAll, at.len, rr[q]);
-      rlen[q] = todo ? len : 0;
-      rfl[q] = __shfl_sync(kAll, at.fl, rr[q]);
-      rown[q] = __shfl_sync(kAll, own_slot, rr[q]);
-      todo &= todo - 1;
-    }
-    const int most = max(max(rlen[0], rlen[1]), max(rlen[2], rlen[3]));
-    for (int s = lane; s < most; s += 32) {
-      uint32_t m[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int w = rlo[q] + s;
-        m[q] = s < rlen[q] ? ((rfl[q] & 1) ? 1u : (__ldg(a.mask + (w >> 5)) >> (w & 31)) & 1u) : 0u;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (m[q]) acc[rr[q] * a.stride + s] = (rfl[q] & 1) && s == rown[q] ? a.diagonal : 0.0;
-    }
-  }
-  __syncwarp();
-  const int len0 = __shfl_sync(kAll, at.len, first);
-  if (a.zero && len0 > 0 && __all_sync(kAll, at.len == len0 || !((mine >> lane) & 1u))) {
-    // rows of one length: the lanes go through their entries without a gap
-    const int jump = 32 / len0, rest = 32 - jump * len0, end = (first + count) * len0, pad = a.stride - len0;
-    // entry t of the group stands at value index t + delta of its row
-    const int delta = at.lo - lane * len0;
-    int rr = lane / len0, s = lane - rr * len0;
-    rr += first;
-    const double* from = acc + first * len0 + lane;
-#pragma unroll 4
-    for (int t = first * len0 + lane; t < end + lane; t += 32, from += 32) {
-      const int to = t + __shfl_sync(kAll, delta, rr);
-      if (t < end) a.values[to] = from[rr * pad];
-      s += rest;
-      const bool wrap = s >= len0;
-      if (wrap) s -= len0;
-      rr += wrap ? jump + 1 : jump;
-    }
-    return;
-  }
-#pragma unroll 4
-  for (int rr = first; rr < first + count; ++rr) {
-    const int rlo = __shfl_sync(kAll, at.lo, rr), rlen = __shfl_sync(kAll, at.len, rr);
-    const double* seg = acc + rr * a.stride;
-    for (int s = lane; s < rlen; s += 32) {
-      const double v = seg[s];
-      if (a.zero) a.values[rlo + s] = v;
-      else a.values[rlo + s] += v;
-    }
-  }
-}
-
 // One warp a CTA: a finished warp's shared memory goes to the next one at once
 // (P2 n=96: 1.15 ms against 1.22 ms with CTAs of two and four warps).
 // CTAs per SM to fit in registers (fewer registers spill, more leave too few
 // warps):
 constexpr int kMinV1 = 20, kMinV2 = 13, kMinE = 20, kMinE3 = 16, kMinF3 = 20;
-
-// The kernels of one call write different rows: the later one starts while
-// the earlier one runs (programmatic dependent launch) and ends after it, so
-// that what follows in the stream waits for both.
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void end_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 
 // Vertex rows (P1: all rows): the cells around vertex a as strips, each with
 // its three other vertices p, q, r, where r is fetched and p, q are two of
@@ -1342,16 +1220,9 @@ __global__ void __launch_bounds__(32, kMinF3) k_rows_f3(const WalkArgs a) {
   end_after_previous();
 }
 
-unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
-
 int odd_at_least(int n) { return n | 1; }
 
 size_t segment_bytes(int stride) { return sizeof(double) * 32 * (size_t)stride; }
-
-template <typename K>
-void raise_smem(K kernel) {
-  FE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSm));
-}
 
 int degree_of(int kind) {
   switch (kind) {
@@ -1373,20 +1244,6 @@ void raise_p3_of() {
 void raise_p3() {
   raise_p3_of<FE_COEFF_CONSTANT>();
   raise_p3_of<FE_COEFF_DG0>();
-}
-
-void exclusive_scan(int32_t* v, int64_t n, cudaStream_t s) {
-  size_t tb = 0;
-  FE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, v, v, (int)n, s));
-  DevBuf<unsigned char> tmp(std::max<size_t>(1, tb));
-  FE_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, v, v, (int)n, s));
-  FE_CUDA(cudaStreamSynchronize(s));
-}
-
-bool capturing(cudaStream_t s) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  FE_CUDA(cudaStreamIsCapturing(s, &st));
-  return st != cudaStreamCaptureStatusNone;
 }
 
 // a P1 coefficient's dofmap is the mesh's own vertex numbering (then its
@@ -1615,22 +1472,6 @@ bool rows_supported(fe_form_s& f, const fe_bc_s* bc0, const fe_bc_s* bc1, cudaSt
 }
 
 namespace {
-// `beside`: the kernel before it in the stream is one of this call's
-template <typename K>
-void launch_beside(K kernel, unsigned grid, size_t smem, bool beside, const WalkArgs& a, cudaStream_t s) {
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(32);
-  c.dynamicSmemBytes = smem;
-  c.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = &at;
-  c.numAttrs = beside ? 1 : 0;
-  FE_CUDA(cudaLaunchKernelEx(&c, kernel, a));
-}
-
 template <int DEG, int COEF>
 void launch_parts(const fe_form_s& f, WalkArgs a, cudaStream_t s) {
   const fe_form_s::RowsPlan& P = *f.rows_plan;
@@ -1711,31 +1552,8 @@ void assemble_matrix_rows(fe_form_s& f, double* values, const fe_bc_s* bc, doubl
   const Coefficient& k = f.coeff[0];
   a.coef = k.values;
   a.coef_const = k.kind < 0 ? 1.0 : k.constant[0];
-  a.row_ptr = sp.row_ptr.p;
-  a.zero = zero ? 1 : 0;
   a.values = values;
-  bool set_diag = false;
-  if (bc) {
-    // which rows a BC touches: once per (pattern, BC), as the diagonal slots of the zero pass
-    auto& F = bc->row_flags[sp.id];
-    if (!F) {
-      auto t = std::make_unique<fe_bc_s::RowFlags>();
-      t->flags.alloc((size_t)std::max<int64_t>(1, sp.num_rows));
-      t->mask.alloc((size_t)(sp.nnz / 32 + 1));
-      if (sp.nnz) k_rows_bc_mask<<<blocks_for(sp.nnz, 256), 256, 0, s>>>(sp.col.p, sp.nnz, bc->markers.p, t->mask.p);
-      k_rows_bc_flags<<<blocks_for(sp.num_rows, 256), 256, 0, s>>>(sp.row_ptr.p, sp.num_rows, bc->markers.p,
-                                                                   t->mask.p, t->flags.p);
-      FE_CUDA(cudaGetLastError());
-      FE_CUDA(cudaStreamSynchronize(s));  // calls on other streams may read them next
-      F = std::move(t);
-    }
-    a.flags = F->flags.p;
-    a.mask = F->mask.p;
-    // the marked rows are the owned listed ones: their diagonal goes with the rows
-    const bool owned = bc->markers_are_dofs && bc->n_owned == bc->n_bc;
-    a.diagonal = owned && zero ? diagonal : 0.0;
-    set_diag = !owned || !zero;
-  }
+  const bool set_diag = set_bc_rows(a, sp, bc, diagonal, zero, s);
   const int kind = k.kind < 0 ? FE_COEFF_CONSTANT : k.kind;
   if (f.kind == FE_FORM_P3_STIFFNESS) {
     if (kind == FE_COEFF_DG0) launch_p3<FE_COEFF_DG0>(f, a, s);

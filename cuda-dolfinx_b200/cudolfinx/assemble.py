@@ -145,12 +145,14 @@ class CUDAAssembler:
         """Assemble a bilinear form into a device CSR matrix (not finalised).
 
         ``variant``: "auto" (the row walk for FP64 P1 stiffness from 98,304
-        cells and P2 from 65,536 cells on and for FP64 P3, where it applies; else the block
+        cells and P2 from 65,536 cells on, for FP64 P3 and for FP32 vector-P2
+        elasticity, where it applies; else the block
         variant for P1 on meshes of >= 2^20 cells, coalesced scatter for P2
         stiffness, vector-P2 elasticity and FP64 P3 stiffness, atomic scatter
         otherwise),
-        "row-walk" (FP64 P1/P2/P3 stiffness: one thread per row walks the cells
-        around its node; bitwise reproducible; not offered for two different
+        "row-walk" (FP64 P1/P2/P3 stiffness, FP32 vector-P2 elasticity: the
+        cells around a row's node are added up by the row's own thread or warp;
+        bitwise reproducible; not offered for two different
         spaces or BCs, block patterns, dofs shared between several vertices
         or overlapping cells),
         "deterministic" (bitwise reproducible: ordered tile gather for P1/P2,

@@ -26,11 +26,13 @@ from .la import CUDAMatrix
 CANDIDATES = {
     "P1_STIFFNESS": ("atomic", "block", "tile", "row-walk"),
     "P2_STIFFNESS": ("atomic", "block", "grouped", "coalesced", "row-walk"),
-    "VP2_ELASTICITY": ("coalesced", "atomic", "atomic-full"),
-    "P3_STIFFNESS": ("coalesced", "atomic", "row-walk"),  # coalesced, row-walk: FP64 element tensors only (skipped for FP32)
+    "VP2_ELASTICITY": ("coalesced", "atomic", "atomic-full", "row-walk"),
+    "P3_STIFFNESS": ("coalesced", "atomic", "row-walk"),  # coalesced: FP64 element tensors only (skipped for FP32)
 }
-# the row walk is timed from the sizes on where it is the engine's default
-ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536, "P3_STIFFNESS": 0}
+# the row walk is timed from the sizes on where it is the engine's default,
+# for the precision of the element tensors that it takes
+ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536, "P3_STIFFNESS": 0, "VP2_ELASTICITY": 0}
+ROW_WALK_PRECISION = {"P1_STIFFNESS": "fp64", "P2_STIFFNESS": "fp64", "P3_STIFFNESS": "fp64", "VP2_ELASTICITY": "fp32"}
 # launch shapes of the atomic scatter timed per form kind: (cells per CTA,
 # byte maps staged in shared memory)
 LAUNCHES = {
@@ -73,7 +75,7 @@ class VariantTuner:
         # for constant and cellwise coefficients
         field = any(getattr(getattr(c, "function_space", None), "degree", 0) for c in a._spec.coefficients)
         for v in CANDIDATES.get(a._spec.kind, ("atomic",)):
-            if v == "row-walk" and (field or a._spec.precision != "fp64"
+            if v == "row-walk" and (field or a._spec.precision != ROW_WALK_PRECISION[a._spec.kind]
                                     or a._spec.mesh.num_cells < ROW_WALK_CELLS[a._spec.kind]):
                 continue
             shapes = LAUNCHES.get(a._spec.kind, ((0, 1),)) if v in ("atomic", "atomic-full") else ((0, 1),)

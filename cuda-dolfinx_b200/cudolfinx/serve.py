@@ -92,12 +92,13 @@ def problem_sizes(kind: str, n: int) -> dict:
 
 def slot_bytes(kind: str, n: int) -> int:
     """Device bytes of one slot: CSR values, cell-to-slot map, row-walk plan
-    (records of 12 or 20 bytes for a cell's rows, padded, and per row), b, x,
+    (records of 12, 16 or 20 bytes for a cell's rows, padded, and per row), b, x,
     BC data, solver scratch (6 vectors, an FP32 copy of the values and, for vector P2,
     its block-column index), coefficients."""
     s = problem_sizes(kind, n)
     ncoef = 2 if kind == "vp2" else 1
-    walk = {"p1": 60 * s["cells"] + 16 * s["rows"], "p2": 240 * s["cells"] + 16 * s["rows"], "vp2": 0}[kind]
+    walk = {"p1": 60 * s["cells"] + 16 * s["rows"], "p2": 240 * s["cells"] + 16 * s["rows"],
+            "vp2": 176 * s["cells"] + 8 * s["rows"]}[kind]
     return (8 * s["nnz"] + s["cells"] * s["k"] * s["k"] + walk + 8 * 2 * s["rows"] + 9 * s["rows"] + 8 * 6 * s["rows"]
             + 4 * s["nnz"] + (s["nnz"] // 9 * 4 + s["rows"] // 3 * 4 if kind == "vp2" else 0)
             + 8 * ncoef * s["cells"])

@@ -127,7 +127,7 @@ enum fe_precision {
                                      reduction per slot (falls back to the atomic scatter when the
                                      mesh's groups share no structure)                                */
 #define FE_ASM_COALESCED 512u     /* P2 stiffness, vector-P2 elasticity, FP64 P3 stiffness (the default
-                                     for each): the warp's reductions issued row by row (consecutive
+                                     for each where the row walk is not): the warp's reductions issued row by row (consecutive
                                      lanes on one cell's CSR row, so an instruction's reductions
                                      share L2 sectors); FE_ASM_ATOMIC keeps one thread's reductions
                                      per cell                                                       */
@@ -135,7 +135,8 @@ enum fe_precision {
                                      the row's node and stores the row once, without reductions or a
                                      zero pass (reproducible); the default from 98,304 (P1) and 65,536
                                      (P2) cells on and for P3, below which the call asks for it by this flag; needs
-                                     one space and one set of BCs for rows and columns               */
+                                     one space and one set of BCs for rows and columns.  FP32 vector-P2
+                                     elasticity (its default): a warp walks three nodes' cells        */
 
 /* ---- errors / context --------------------------------------------------- */
 const char* fe_last_error(void);
