@@ -524,8 +524,8 @@ __global__ void __launch_bounds__(kBlockP3) k_mat_p3_atomic(const MatArgs a) {
 
 // ---------------------------------------------------------------------------
 // P3 stiffness (cellwise-constant coefficient, FP64) with the reductions
-// coalesced per warp ("coalesced" variant, the FP64 P3 default).  The
-// 210-entry element tensor is too large to stage per cell, so each thread
+// coalesced per warp ("coalesced" variant, the FP64 P3 default where the row
+// walk does not apply).  The 210-entry element tensor is too large to stage per cell, so each thread
 // computes only its cell's geometry, g[s] = k * Ghat_s (6 doubles), row
 // starts and column masks; the warp then walks its 32 cells and evaluates
 // the 400 entries of each in 13 rounds, lane l of round r on entry
@@ -692,12 +692,13 @@ __global__ void __launch_bounds__(kBlock) k_mat_vp2_atomic(const MatArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Vector-P2 elasticity with the reductions coalesced per warp (the vector-P2
-// default).  Entry (row (i,a), column (j,b)) of the 30x30 element matrix is
+// Vector-P2 elasticity with the reductions coalesced per warp (the default of
+// FP64 vector P2 and of FP32 up to 196,608 cells).
+// Entry (row (i,a), column (j,b)) of the 30x30 element matrix is
 // sum_pq C_ij^pq W^ab_pq with C_ij^pq = int_ref d_p phi_i d_q phi_j (the
 // table kP2GradGrad) and W^ab the 9 geometric weights of component block
 // (a, b) (elasticity_weights).  One thread per cell computes the 6 weight
-// blocks a <= b into shared memory; the warp then walks its 32 cells: one
+// blocks a <= b into shared memory; the warp then walks its CW cells: one
 // instruction per element row (i, a), lane 3j + b on column (j, b), so the
 // 30 reductions land on the 10 consecutive slot triples of one CSR row
 // (~2 per 32-byte sector, against 1 for the thread-per-cell scatter) and no
@@ -711,9 +712,9 @@ __global__ void __launch_bounds__(kBlock) k_mat_vp2_atomic(const MatArgs a) {
 // ---------------------------------------------------------------------------
 constexpr int kVCoalThreads = 64;
 
-template <typename T>
+template <typename T, int CW>
 __global__ void __launch_bounds__(kVCoalThreads) k_mat_vp2_coal(const MatArgs a) {
-  constexpr int NT = kVCoalThreads;
+  constexpr int NT = kVCoalThreads / 32 * CW;  // cells of the CTA
   constexpr bool kRowSums = sizeof(T) == 4;
   __shared__ T sC[900];
   __shared__ T sW[NT * 54];                         // per cell: blocks (00,11,22,01,02,12) x 9
@@ -721,12 +722,12 @@ __global__ void __launch_bounds__(kVCoalThreads) k_mat_vp2_coal(const MatArgs a)
   __shared__ int32_t srp[NT * 10];                  // scalar row 3R of local node i (component 0)
   __shared__ int32_t sL[NT * 10];                   // its length (the rows 3R+1, 3R+2 follow)
   __shared__ uint32_t smr[NT], smc[NT];             // masked rows / columns, bit 3i + component
-  const int tid = threadIdx.x, lane = tid & 31, w0 = tid & ~31;
-  for (int t = tid; t < 900; t += NT) sC[t] = (T)kP2GradGrad[t];
+  const int tid = threadIdx.x, lane = tid & 31, w0 = (tid >> 5) * CW, own = w0 + lane;
+  for (int t = tid; t < 900; t += kVCoalThreads) sC[t] = (T)kP2GradGrad[t];
   const int64_t c0 = blockIdx.x * (int64_t)NT;
   const int64_t left = a.num_cells - c0;
   const int ncell = left < NT ? (int)left : NT;
-  const int wcells = ncell - w0 < 0 ? 0 : (ncell - w0 < 32 ? ncell - w0 : 32);
+  const int wcells = ncell - w0 < 0 ? 0 : (ncell - w0 < CW ? ncell - w0 : CW);
   {
     // each warp stages its own cells' byte maps ((c0 + w0) * 100 is a multiple of 16)
     const uint4* src = reinterpret_cast<const uint4*>(a.pos + (c0 + w0) * 100);
@@ -734,8 +735,8 @@ __global__ void __launch_bounds__(kVCoalThreads) k_mat_vp2_coal(const MatArgs a)
     const int nvec = (wcells * 100 + 15) / 16;
     for (int t = lane; t < nvec; t += 32) dst[t] = __ldg(src + t);
   }
-  if (tid < ncell) {
-    const int64_t c = c0 + tid;
+  if (lane < wcells) {
+    const int64_t c = c0 + own;
     CellGeo g;
     cell_geometry(a.x, load_geom(a.geom, c), g);
     const double lam = coef_cell(a.c0, c), mu = coef_cell(a.c1, c);
@@ -743,7 +744,7 @@ __global__ void __launch_bounds__(kVCoalThreads) k_mat_vp2_coal(const MatArgs a)
     for (int blk = 0; blk < 6; ++blk) {  // rolled: unrolled it takes 144 registers (FP32) instead of 108
       const int ca = blk < 3 ? blk : (blk == 5 ? 1 : 0);
       const int cb = blk < 3 ? blk : (blk == 3 ? 1 : 2);
-      elasticity_weights<T>(g, lam, mu, ca, cb, sW + tid * 54 + blk * 9);
+      elasticity_weights<T>(g, lam, mu, ca, cb, sW + own * 54 + blk * 9);
     }
     const int32_t* d0 = a.dofs0 + c * 10;
     const int32_t* d1 = a.dofs1 + c * 10;
@@ -753,16 +754,16 @@ __global__ void __launch_bounds__(kVCoalThreads) k_mat_vp2_coal(const MatArgs a)
       // masked rows / columns: BC dofs and nodes outside a restriction (-1)
       const int R = __ldg(d0 + i), C = __ldg(d1 + i);
       const int32_t r0 = R < 0 ? 0 : __ldg(a.row_ptr + 3 * R);
-      srp[tid * 10 + i] = r0;
-      sL[tid * 10 + i] = R < 0 ? 0 : __ldg(a.row_ptr + 3 * R + 1) - r0;
+      srp[own * 10 + i] = r0;
+      sL[own * 10 + i] = R < 0 ? 0 : __ldg(a.row_ptr + 3 * R + 1) - r0;
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         mr |= (R < 0 || (a.bc0 && __ldg(a.bc0 + 3 * R + q)) ? 1u : 0u) << (3 * i + q);
         mc |= (C < 0 || (a.bc1 && __ldg(a.bc1 + 3 * C + q)) ? 1u : 0u) << (3 * i + q);
       }
     }
-    smr[tid] = mr;
-    smc[tid] = mc;
+    smr[own] = mr;
+    smc[own] = mc;
   }
   __syncthreads();  // the C table; the warp's own cells need only their warp
   // lanes 30 and 31 run along (the shuffles below take the whole warp) on
@@ -1959,8 +1960,19 @@ void launch_matrix_atomic(const MatLaunch& L, cudaStream_t s) {
     }
     case FE_FORM_VP2_ELASTICITY:
       if (L.coalesced && !a.upper) {
-        auto k = f32 ? k_mat_vp2_coal<float> : k_mat_vp2_coal<double>;
-        k<<<grid_for(L.num_cells, kVCoalThreads), kVCoalThreads, 0, s>>>(a);
+        auto go = [&](auto width) {
+          constexpr int CW = decltype(width)::value;
+          auto k = f32 ? k_mat_vp2_coal<float, CW> : k_mat_vp2_coal<double, CW>;
+          k<<<grid_for(L.num_cells, kVCoalThreads / 32 * CW), kVCoalThreads, 0, s>>>(a);
+        };
+        // cells a warp walks (FP64 / FP32, us per call on B200 with 32, 16, 8, 4): n=5 84, 49, 33, 28 / 126, 72,
+        // 43; n=12 93, 64, 49, 51 / 133, 82, 55; n=20 239, 174, 167, 183 / 185, 202, 167; n=26 387, 343, 341, 380 /
+        // 450, 430, 327; n=32 705, 593, 609, 687 / 722, 724, 574; n=44 1,718, 1,526, 1,546 / 1,964, 1,927, 1,510:
+        // a short walk for meshes that leave schedulers idle, else the shared memory of few cells, which lets more
+        // warps in
+        if (L.num_cells <= 4736) go(std::integral_constant<int, 4>{});  // 148 SMs x 4 schedulers x 2 warps x 4 cells
+        else if (f32 || L.num_cells < 131072) go(std::integral_constant<int, 8>{});
+        else go(std::integral_constant<int, 16>{});
       } else if (f32) {
         k_mat_vp2_atomic<float><<<grid, kBlock, 0, s>>>(a);
       } else {

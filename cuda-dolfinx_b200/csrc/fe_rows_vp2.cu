@@ -14,10 +14,10 @@
 // instructions a step, 2,125 us at n=44).
 //
 // Measured (us per call, this walk / the warp-coalesced scatter): n=44 1,328 /
-// 1,951, n=32 575 / 719, n=26 361 / 448, n=20 183 / 184, n=16 113 / 150, n=12
-// 68 / 133, n=5 31 / 125; so it is taken at every size.  FP64 tensors take
-// twice the shared memory and gain nothing on large meshes (n=44 1,693 /
-// 1,698, n=32 704 / 690, n=16 130 / 117): they keep the scatter.  Bound by
+// 1,510, n=32 575 / 574, n=26 361 / 327, n=20 183 / 167, n=12 68 / 55, n=5 31 /
+// 30; so it is the default from 196,608 cells (n=32) on.  FP64 tensors take
+// twice the shared memory and are slower at every size (n=44 1,693 / 1,526,
+// n=32 704 / 593): they keep the scatter.  Bound by
 // shared-memory wavefronts (55-58 % of the pipe: 190 a step, half of them the
 // block's nine adds into its columns, whose banks meet) and by latency at ten
 // warps an SM, which the segments leave room for; evaluating the next step's
@@ -433,7 +433,7 @@ void launch_vp2(const fe_form_s& f, VWalkArgs a, cudaStream_t s) {
 void reset_nodes_plan(fe_form_s& f) { f.nodes_plan.reset(); }
 
 bool vp2_rows_default(const fe_form_s& f) {
-  return f.kind == FE_FORM_VP2_ELASTICITY && f.precision == FE_PREC_FP32;
+  return f.kind == FE_FORM_VP2_ELASTICITY && f.precision == FE_PREC_FP32 && f.mesh && f.mesh->num_cells >= 196608;
 }
 
 // Builds the plan of an elasticity form bound to a plain pattern, or leaves

@@ -146,7 +146,7 @@ class CUDAAssembler:
 
         ``variant``: "auto" (the row walk for FP64 P1 stiffness from 98,304
         cells and P2 from 65,536 cells on, for FP64 P3 and for FP32 vector-P2
-        elasticity, where it applies; else the block
+        elasticity from 196,608 cells on, where it applies; else the block
         variant for P1 on meshes of >= 2^20 cells, coalesced scatter for P2
         stiffness, vector-P2 elasticity and FP64 P3 stiffness, atomic scatter
         otherwise),

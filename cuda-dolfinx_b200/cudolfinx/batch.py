@@ -31,7 +31,7 @@ CANDIDATES = {
 }
 # the row walk is timed from the sizes on where it is the engine's default,
 # for the precision of the element tensors that it takes
-ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536, "P3_STIFFNESS": 0, "VP2_ELASTICITY": 0}
+ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536, "P3_STIFFNESS": 0, "VP2_ELASTICITY": 196608}
 ROW_WALK_PRECISION = {"P1_STIFFNESS": "fp64", "P2_STIFFNESS": "fp64", "P3_STIFFNESS": "fp64", "VP2_ELASTICITY": "fp32"}
 # launch shapes of the atomic scatter timed per form kind: (cells per CTA,
 # byte maps staged in shared memory)

@@ -98,7 +98,7 @@ def slot_bytes(kind: str, n: int) -> int:
     s = problem_sizes(kind, n)
     ncoef = 2 if kind == "vp2" else 1
     walk = {"p1": 60 * s["cells"] + 16 * s["rows"], "p2": 240 * s["cells"] + 16 * s["rows"],
-            "vp2": 176 * s["cells"] + 8 * s["rows"]}[kind]
+            "vp2": 176 * s["cells"] + 8 * s["rows"] if s["cells"] >= 196608 else 0}[kind]
     return (8 * s["nnz"] + s["cells"] * s["k"] * s["k"] + walk + 8 * 2 * s["rows"] + 9 * s["rows"] + 8 * 6 * s["rows"]
             + 4 * s["nnz"] + (s["nnz"] // 9 * 4 + s["rows"] // 3 * 4 if kind == "vp2" else 0)
             + 8 * ncoef * s["cells"])

@@ -136,7 +136,8 @@ enum fe_precision {
                                      zero pass (reproducible); the default from 98,304 (P1) and 65,536
                                      (P2) cells on and for P3, below which the call asks for it by this flag; needs
                                      one space and one set of BCs for rows and columns.  FP32 vector-P2
-                                     elasticity (its default): a warp walks three nodes' cells        */
+                                     elasticity (the default from 196,608 cells on): a warp walks three
+                                     nodes' cells                                                     */
 
 /* ---- errors / context --------------------------------------------------- */
 const char* fe_last_error(void);

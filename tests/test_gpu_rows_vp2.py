@@ -1,4 +1,4 @@
-"""The row walk of FP32 vector-P2 elasticity (variant "row-walk", its default)
+"""The row walk of FP32 vector-P2 elasticity (variant "row-walk")
 against the warp-coalesced scatter (variant "coalesced").
 
 Both add the same element entries, rounded to FP32 alike, in FP64: an entry's
@@ -35,7 +35,7 @@ def _form(n, order, coef, cells=None):
 
 @pytest.mark.parametrize("coef", ["const", "dg0"])
 @pytest.mark.parametrize("n,order,cells", [(1, "natural", None), (1, "natural", [0]), (1, "permuted", [0, 3]), (2, "permuted", None),
-                                           (5, "natural", None), (5, "permuted", None), (9, "natural", None)])
+                                           (5, "natural", None), (5, "permuted", None), (9, "natural", None), (11, "natural", None)])
 def test_walk_matches_scatter(n, order, cells, coef):
     ensure_library()
     import cudolfinx as cx
