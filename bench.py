@@ -90,21 +90,36 @@ L2_BYTES = 126 * 1024 * 1024
 VECTOR_KERNELS = 3
 
 
-def matrix_kernels(kind: str, variant: str, big: bool = False, nnz: int = 1 << 30) -> int:
-    """Kernel launches of one fe_assemble_matrix call (with BCs): 2 for the
-    single-pass variants (row gather, tile, ordered tile: kernel +
-    set_diagonal) and for the scatters after the zero pass that also writes
-    the BC diagonal (coalesced, block, atomic with both reductions: zero +
-    kernel), 3 with the upper-triangle scatter (zero + scatter + transpose
-    pass) and for the sorted-slot reduction (element tensors + gather +
-    set_diagonal)."""
+def default_variant(kind: str, precision: str, cells: int) -> str:
+    """The variant "auto" resolves to (fe_assemble_matrix's default) on a plain
+    pattern with constant or cellwise coefficients: the row walk for FP64 P1
+    from 98,304 cells, P2 from 65,536 cells and P3, and for FP32 vector-P2
+    elasticity from 196,608 cells; else the block kernel for P1 meshes of >= 2^20 cells, the
+    coalesced scatter for P2, vector P2 and FP64 P3, the atomic scatter otherwise."""
+    walk = {"p1": 98304, "p2": 65536, "p3": 0} if precision == "fp64" else {"vp2": 196608}
+    if cells >= walk.get(kind, 1 << 62):
+        return "row-walk"
+    if kind == "p1" and cells >= 1 << 20:
+        return "block"
+    return "coalesced" if kind in ("p2", "vp2") or (kind == "p3" and precision == "fp64") else "atomic"
+
+
+def matrix_kernels(kind: str, variant: str) -> int:
+    """Kernel launches of one fe_assemble_matrix call (with BCs) by a resolved
+    variant: 1 to 3 for the row walk (one per kind of node; vector P2: vertices
+    and edge nodes), 2 for the single-pass variants (row gather, tile, ordered
+    tile: kernel + set_diagonal) and for the scatters after the zero pass that
+    also writes the BC diagonal (coalesced, block, atomic with both reductions:
+    zero + kernel), 3 with the upper-triangle scatter (zero + scatter +
+    transpose pass) and for the sorted-slot reduction (element tensors + gather
+    + set_diagonal)."""
+    if variant == "row-walk":
+        return {"p1": 1, "p2": 2, "p3": 3, "vp2": 2}[kind]
     if variant in ("tile", "row-gather") or (variant == "deterministic" and kind in ("p1", "p2")):
         return 2
     if variant in ("sorted-slot", "deterministic"):
         return 3
-    atomic = variant == "atomic" or (variant == "auto" and not (kind == "p1" and big)
-                                     and kind not in ("p2", "vp2", "p3"))
-    if kind in ("p1", "vp2", "p3") and atomic:
+    if kind in ("p1", "vp2", "p3") and variant == "atomic":
         return 3  # zero + upper-triangle scatter + lower-triangle transpose
     return 2  # zero (with the BC diagonal) + kernel
 
@@ -603,15 +618,9 @@ def run_gpu(args, rank, world, local_rank):
         pass
     peak = peaks.get("hbm_gbs", 6650.0)
     achieved = alg / (mat_ms / 1e3) / 1e9
-    # the variant "auto" resolves to (fe_assemble_matrix's default): the block
-    # kernel for P1 meshes of >= 2^20 cells, the coalesced scatter for P2
-    # stiffness, vector-P2 elasticity and FP64 P3 stiffness, the atomic
-    # scatter otherwise
     resolved = args.variant
     if resolved == "auto":
-        resolved = ("block" if (W["kind"] == "p1" and len(I["cells"]) >= (1 << 20))
-                    else "coalesced" if (W["kind"] in ("p2", "vp2") or (W["kind"] == "p3" and W["precision"] == "fp64"))
-                    else "atomic")
+        resolved = default_variant(W["kind"], W["precision"], len(I["cells"]))
     kernel_key = f"{args.workload}:{resolved}"
     traffic = load_traffic(kernel_key)
     out = {
@@ -638,7 +647,7 @@ def run_gpu(args, rank, world, local_rank):
                      if "hbm_gbs" in peaks else "fallback 6650 GB/s"},
         "matrix_nnz_per_s": nnz / (mat_ms / 1e3),
         "rhs_ms": rhs_ms,
-        "gpu_launches": (matrix_kernels(W["kind"], args.variant, len(I["cells"]) >= (1 << 20), nnz)
+        "gpu_launches": (matrix_kernels(W["kind"], resolved)
                          + VECTOR_KERNELS + (args.rhs == "calls"))
         * args.steps,
         "clocks": clk,
@@ -1542,8 +1551,11 @@ def run_gpu_multimesh(args, rank, world, local_rank):
         pass
     peak = peaks.get("hbm_gbs", 6650.0)
     achieved = alg / (ms / 1e3) / 1e9
-    launches = sum(matrix_kernels(I["kind"], it["variant"], len(I["cells"]) >= (1 << 20), item[1].sparsity.nnz)
-                   for I, item, it in zip(Is, items, G.items))
+    launches = 0
+    for I, it in zip(Is, G.items):
+        v = it["variant"]
+        launches += matrix_kernels(I["kind"], default_variant(I["kind"], it["a"]._spec.precision, len(I["cells"]))
+                                   if v == "auto" else v)
     chosen = {}
     for it in G.items:
         chosen[it["variant"]] = chosen.get(it["variant"], 0) + 1
@@ -1660,10 +1672,17 @@ def serve_working_set(kind, n, solver="fp64"):
     return per_nnz * sz["nnz"] + (4 + 6 * 8) * sz["rows"]
 
 
-def serve_launches(iterations):
-    # matrix (zero, kernel, diagonal) + right-hand side (zero, lifting, vector with set_bc) + PCG (2 + 80 per 16
-    # iterations)
-    return 3 + 3 + 2 + 80 * ((iterations + 16) // 16)
+def serve_launches(r):
+    # matrix (its kernels; the zero pass counts in them) + right-hand side (zero, lifting, vector with set_bc) + PCG:
+    # 3 and two kernels an iteration, in batches of 8, up to 6 M nonzeros; else 2 and five an iteration in batches of 16
+    from cudolfinx import serve
+
+    sz = serve.problem_sizes(r.kind, r.n)
+    precision = "fp64" if r.kind == "p1" else "fp32"
+    matrix = matrix_kernels(r.kind, default_variant(r.kind, precision, sz["cells"]))
+    if r.kind != "vp2" and sz["nnz"] <= 6000000:
+        return matrix + 3 + 3 + 16 * ((r.iterations + 8) // 8)
+    return matrix + 3 + 2 + 80 * ((r.iterations + 16) // 16)
 
 
 def run_gpu_serve(args, rank, world, local_rank):
@@ -1777,7 +1796,7 @@ def run_gpu_serve(args, rank, world, local_rank):
                      "note": "bytes of the requests whose PCG working set (values, columns, vectors) fits in the "
                              "126 MB L2 are served from L2 on every iteration after the first; that share "
                              "(l2_resident_share) can lift the fraction of HBM above 1"},
-        "gpu_launches": sum(serve_launches(r.iterations) for r in served_results if r.error is None),
+        "gpu_launches": sum(serve_launches(r) for r in served_results if r.error is None),
         "e2e": {"value": top["throughput_rps"], "unit": "req/s",
                 "h2d_bytes_per_step": int(np.mean([8 * sum(c.size for c in r.coef) for r in base])),
                 "d2h_bytes_per_step": int(np.mean([8 * serve.problem_sizes(r.kind, r.n)["rows"] for r in base])),
@@ -1921,7 +1940,7 @@ def main():
     ap.add_argument("--workload", choices=sorted(WORKLOADS) + ["batch", "multimesh", "serve", "blocksys", "interp", "dg"],
                     default="p2")
     ap.add_argument("--variant", choices=["auto", "tile", "atomic", "atomic-full", "sorted-slot", "deterministic",
-                                          "row-gather", "block", "grouped", "coalesced"], default="auto")
+                                          "row-gather", "block", "grouped", "coalesced", "row-walk"], default="auto")
     ap.add_argument("--seed", type=int, default=0)
     ap.add_argument("--graph-branches", type=int, default=8,
                     help="multimesh: parallel branches of the captured graph (independent meshes overlap)")
