@@ -33,6 +33,18 @@ CANDIDATES = {
 # for the precision of the element tensors that it takes
 ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536, "P3_STIFFNESS": 0, "VP2_ELASTICITY": 196608}
 ROW_WALK_PRECISION = {"P1_STIFFNESS": "fp64", "P2_STIFFNESS": "fp64", "P3_STIFFNESS": "fp64", "VP2_ELASTICITY": "fp32"}
+# FP32 element tensors: variants of one tuple round an entry alike, those of the
+# other tuple differently (5e-9 of the largest entry for P2, 5e-8 for vector P2),
+# so the tuple is chosen by size and only its members are timed: the values do
+# not depend on a measurement.  (cells, variants below, variants from there on);
+# below: the faster ones when the line was drawn, us atomic / coalesced, P2 n=14
+# 19.4 / 21.4, n=15 (20,250 cells) 21.5 / 21.5, n=16 23.5 / 21.5; vector P2 n=16
+# 115 / 152, n=18 (34,992) 158 / 161, n=19 218 / 177.  The vector-P2 scatter has
+# become faster since (n=4 28 us, atomic 58); the line stays, as its values do.
+FP32_VARIANTS = {
+    "P2_STIFFNESS": (22000, ("atomic",), ("block", "grouped", "coalesced")),
+    "VP2_ELASTICITY": (38000, ("atomic",), ("coalesced", "row-walk")),
+}
 # launch shapes of the atomic scatter timed per form kind: (cells per CTA,
 # byte maps staged in shared memory)
 LAUNCHES = {
@@ -45,8 +57,10 @@ class VariantTuner:
     """Chooses the fastest matrix variant per (form kind, precision, size
     class) and, for the atomic scatter, its launch shape (cells per CTA and
     shared-memory staging of the byte maps); size classes are powers of two of
-    the cell count.  ``choose`` returns the variant name and leaves the
-    chosen launch shape set on the form."""
+    the cell count, and the first mesh of a class decides for it.  For FP32
+    element tensors the candidates are the variants that round alike
+    (FP32_VARIANTS), so that no timing decides a value.  ``choose`` returns
+    the variant name and leaves the chosen launch shape set on the form."""
 
     def __init__(self, reps: int = 3):
         self.reps = reps
@@ -59,6 +73,13 @@ class VariantTuner:
         coef = tuple(type(c).__name__ + (str(c.function_space.degree) if hasattr(c, "function_space") else "")
                      for c in a._spec.coefficients)
         return (a._spec.kind, a._spec.precision, coef, int(math.log2(max(1, C))))
+
+    @staticmethod
+    def candidates(kind: str, precision: str, cells: int) -> tuple:
+        if precision == "fp32" and kind in FP32_VARIANTS:
+            line, below, above = FP32_VARIANTS[kind]
+            return below if cells < line else above
+        return CANDIDATES.get(kind, ("atomic",))
 
     def choose(self, a: CUDAForm, mat: CUDAMatrix, bc0, bc1) -> str:
         k = self.key(a)
@@ -74,7 +95,7 @@ class VariantTuner:
         # mesh's vertex numbering, which the key does not tell: it is timed
         # for constant and cellwise coefficients
         field = any(getattr(getattr(c, "function_space", None), "degree", 0) for c in a._spec.coefficients)
-        for v in CANDIDATES.get(a._spec.kind, ("atomic",)):
+        for v in self.candidates(a._spec.kind, a._spec.precision, a._spec.mesh.num_cells):
             if v == "row-walk" and (field or a._spec.precision != ROW_WALK_PRECISION[a._spec.kind]
                                     or a._spec.mesh.num_cells < ROW_WALK_CELLS[a._spec.kind]):
                 continue
