@@ -214,6 +214,7 @@ __device__ __forceinline__ float vp2_entry(const float* c, const float* u, float
 __device__ __forceinline__ void store_node(const RowOut& a, double* seg, int lo, int len, int own_slot, int fl,
                                            int lane) {
   const int n = 3 * len;
+  if (n == 0) return;  // a node of no cell, the padding of the last group
   double* out = a.values + lo;
   if (fl == 0 && a.zero) {
     // the segment begins at the range's own 16-byte phase
