@@ -314,7 +314,7 @@ __global__ void k_rows_head(const PlanArgs a, const PartArgs p) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t g32 = t >> 5;
   if (g32 >= p.ngroups) return;
-  int4 own = make_int4(-1, -1, -1, 0);
+  int4 own = make_int4(-1, -1, -1, 0), own2 = make_int4(0, 0, 0, 0);
   int n = 0;
   if (t < p.nrows) {
     const int32_t r = p.rows[t];
@@ -336,24 +336,27 @@ __global__ void k_rows_head(const PlanArgs a, const PartArgs p) {
       const uint32_t w =
           p.kind == KIND_F ? 0u : own_slots(a.deg, p.kind, a.pos + (c * a.k + i) * a.k, i, o);
       const int va = g[o[0]], vb = p.kind == KIND_V ? -1 : g[o[1]];
+      int4 o2 = make_int4(0, 0, 0, 0);
+      if (p.kind == KIND_F) {
+        // a, b, c, ab ba ac ca bc cb, the face
+        const uint8_t* b = a.pos + (c * a.k + i) * a.k;
+        auto B = [&](int j) -> uint32_t { return b[j]; };
+        o2.x = (int)(B(o[0]) | (B(o[1]) << 8) | (B(o[2]) << 16) | (B(p3_edge(o[0], o[1])) << 24));
+        o2.y = (int)(B(p3_edge(o[1], o[0])) | (B(p3_edge(o[0], o[2])) << 8) | (B(p3_edge(o[2], o[0])) << 16) |
+                     (B(p3_edge(o[1], o[2])) << 24));
+        o2.z = (int)(B(p3_edge(o[2], o[1])) | (B(i) << 8));
+      }
       if (q == 0) {
         own.y = va;
         own.z = vb;
         own.w = p.kind == KIND_F ? g[o[2]] : (int)w;
-        if (p.kind == KIND_F) {
-          // a, b, c, ab ba ac ca bc cb, the face
-          const uint8_t* b = a.pos + (c * a.k + i) * a.k;
-          auto B = [&](int j) -> uint32_t { return b[j]; };
-          p.own2[t] = make_int4(
-              (int)(B(o[0]) | (B(o[1]) << 8) | (B(o[2]) << 16) | (B(p3_edge(o[0], o[1])) << 24)),
-              (int)(B(p3_edge(o[1], o[0])) | (B(p3_edge(o[0], o[2])) << 8) | (B(p3_edge(o[2], o[0])) << 16) |
-                    (B(p3_edge(o[1], o[2])) << 24)),
-              (int)(B(p3_edge(o[2], o[1])) | (B(i) << 8)), 0);
-        }
-      } else if (own.y != va || own.z != vb || (uint32_t)own.w != (p.kind == KIND_F ? (uint32_t)g[o[2]] : w)) {
-        *a.fail = 1u;  // one dof, several vertices or edges
+        own2 = o2;
+      } else if (own.y != va || own.z != vb || (uint32_t)own.w != (p.kind == KIND_F ? (uint32_t)g[o[2]] : w) ||
+                 own2.x != o2.x || own2.y != o2.y || own2.z != o2.z) {
+        *a.fail = 1u;  // one dof, several vertices or edges; cells that name a common face's dofs differently
       }
     }
+    if (p.kind == KIND_F) p.own2[t] = own2;
     if (p.kind == KIND_V) {
       if (n > kMaxStar) *a.fail = 1u;
       else if (n > 0) {
@@ -399,6 +402,7 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
   uint64_t used = 0;  // edge rows: cells already listed (all of them below 64)
   int last = -1;      // mesh vertex the next cell around the edge shares
   int fan = -1;       // the vertex its fan began with
+  uint2 begun = make_uint2(0u, 0u), left = make_uint2(0u, 0u);  // edge rows: slots of the fan's first and last vertex
   uint32_t seen[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};  // slots some cell adds to
   uint32_t written[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
   auto mark = [&](uint32_t b) { seen[b >> 5] |= 1u << (b & 31u); };
@@ -559,6 +563,21 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
     auto B = [&](int j) -> uint32_t { return q[j]; };
     for (int j = 0; j < a.k; ++j) mark(B(j));
     p.cell[at] = (int32_t)c;
+    {
+      // the walk adds a cell's entries of vertex d (d ad bd, P3: d ad da bd db abd) to the next cell's of c, at
+      // the end of a closed fan to the first cell's: both cells have to name those dofs alike
+      auto slots_of = [&](int v, int opposite) {
+        if (a.deg == 2) return make_uint2(B(o[v]) | (B(p2_edge(o[0], o[v])) << 8) | (B(p2_edge(o[1], o[v])) << 16), 0u);
+        return make_uint2(B(o[v]) | (B(p3_edge(o[0], o[v])) << 8) | (B(p3_edge(o[v], o[0])) << 16) |
+                              (B(p3_edge(o[1], o[v])) << 24),
+                          B(p3_edge(o[v], o[1])) | (B(16 + o[opposite]) << 8));
+      };
+      const uint2 sc = slots_of(2, 3), sd = slots_of(3, 2);
+      if (flags & kFanBegin) begun = sc;
+      else if (sc.x != left.x || sc.y != left.y) *a.fail = 1u;
+      if ((flags & kFanClosed) && (sd.x != begun.x || sd.y != begun.y)) *a.fail = 1u;
+      left = sd;
+    }
     if (a.deg == 3) {
       // slots: the six of vertex c (c, ac ca bc cb, abc), the six of d, then cd dc acd bcd
       auto E = [&](int x, int y) { return B(p3_edge(o[x], o[y])); };
@@ -1347,8 +1366,9 @@ bool rows_default(const fe_form_s& f) {
 // Builds the plan of a form bound to a plain pattern; leaves the form without
 // one where the walk does not apply (the assembly then takes the scatter):
 // kinds without a row walk, two different spaces, dofs that stand for several
-// mesh vertices or edges (periodic maps), cells with a repeated dof, rows too
-// long for a warp's shared memory, no memory for the records.
+// mesh vertices or edges (periodic maps), cells with a repeated dof, neighbours
+// that do not share the dofs of a common face (slits), rows too long for a
+// warp's shared memory, no memory for the records.
 void build_rows_plan(fe_form_s& f, cudaStream_t s) {
   f.rows_plan.reset();
   const int deg = degree_of(f.kind);
