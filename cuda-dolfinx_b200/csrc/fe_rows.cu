@@ -79,8 +79,8 @@ struct PlanArgs {
   const int32_t* geom;
   const int32_t* dofs;
   const uint8_t* pos;
-  const int32_t* row_ptr;  // first scalar row of block row R at R * bs
-  int bs;
+  const int32_t* row_ptr;
+  const int32_t* diag;     // slot of (r, r) or -1
   int32_t* inc_ptr;
   int32_t* inc;
   unsigned* fail;
@@ -328,6 +328,8 @@ __global__ void k_rows_head(const PlanArgs a, const PartArgs p) {
       inc[s] = v;
     }
     own.x = r;
+    // a node of no cell: its row, in a pattern of the caller's own, may have its diagonal anywhere, or none
+    if (n == 0) own.w = a.diag[r] < 0 ? -1 : a.diag[r] - a.row_ptr[r];
     for (int q = 0; q < n; ++q) {
       int64_t c;
       int i, g[4], o[4];
@@ -830,7 +832,7 @@ __global__ void __launch_bounds__(32 * PARTS, (DEG == 1 ? kMinV1 : kMinV2) / PAR
     eq = er;
     kq = kr;
   }
-  if (own.y >= 0) seg[own.w & 0xff] += diag;
+  if (own.y >= 0) seg[own.w] += diag;
   if constexpr (PARTS > 1) {
     __syncthreads();
     for (int t = threadIdx.x; t < 32 * a.stride; t += 32 * PARTS) {
@@ -842,7 +844,7 @@ __global__ void __launch_bounds__(32 * PARTS, (DEG == 1 ? kMinV1 : kMinV2) / PAR
     __syncthreads();
   }
   constexpr int kRows = 32 / PARTS;
-  store_rows(a, smem, at, own.w & 0xff, lane, part * kRows, kRows);
+  store_rows(a, smem, at, own.w, lane, part * kRows, kRows);
 }
 
 // Edge rows of P2: node ab; the cells around the edge in fans, each with its
@@ -1083,7 +1085,7 @@ __global__ void __launch_bounds__(64 * PARTS) k_rows_v3(const WalkArgs a) {
     eq = er;
   }
   // (the row's own column: added by the inner warp alone)
-  if (own.y >= 0 && !outer) seg[own.w & 0xff] += diag;
+  if (own.y >= 0 && !outer) seg[own.w] += diag;
   __syncthreads();
   if constexpr (PARTS > 1) {
     for (int t = threadIdx.x; t < 32 * a.stride; t += 64 * PARTS) {
@@ -1095,7 +1097,7 @@ __global__ void __launch_bounds__(64 * PARTS) k_rows_v3(const WalkArgs a) {
     __syncthreads();
   }
   constexpr int kRows = 16 / PARTS;
-  store_rows(a, smem, at, own.w & 0xff, lane, (threadIdx.x >> 5) * kRows, kRows);
+  store_rows(a, smem, at, own.w, lane, (threadIdx.x >> 5) * kRows, kRows);
 }
 
 template <int COEF>
@@ -1403,7 +1405,7 @@ void build_rows_plan(fe_form_s& f, cudaStream_t s) {
     a.dofs = V.dofs.p;
     a.pos = f.pos.p;
     a.row_ptr = f.sp->row_ptr.p;
-    a.bs = V.bs;
+    a.diag = f.sp->diag.p;
     a.inc_ptr = cnt.p;
     a.inc = inc.p;
     a.fail = fail.p;

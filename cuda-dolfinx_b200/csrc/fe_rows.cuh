@@ -44,7 +44,8 @@ __device__ __forceinline__ RowAt row_at(const RowOut& a, int row) {
 
 // The warp's 32 row segments (lane l's at acc + l * stride) to their rows.
 // First the segments of rows that a BC touches take their zeros (and a BC row
-// `diagonal` at its own slot), then all rows are stored, or added with zero == 0.
+// `diagonal` at its own slot, -1: it has none), then all rows are stored, or added
+// with zero == 0.
 // A warp takes the `count` rows from `first` on.
 __device__ __forceinline__ void store_rows(const RowOut& a, double* acc, const RowAt& at, int own_slot, int lane,
                                            int first, int count) {

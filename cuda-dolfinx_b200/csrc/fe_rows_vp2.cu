@@ -54,6 +54,7 @@ constexpr int kBatch = 10;  // steps whose weights are formed together: 30 lanes
 struct VPlanArgs {
   int64_t num_cells, num_nodes;
   const int32_t* row_ptr;
+  const int32_t* diag;  // slot of (r, r) or -1
   const int32_t* dofs;  // [cells][10]
   const uint8_t* pos;   // [cells][10][10]
   int32_t* inc_ptr;
@@ -120,7 +121,15 @@ __global__ void k_nodes_head(const VPlanArgs a, const VPartArgs p) {
     own.x = 3 * r;
     own.y = a.row_ptr[3 * r];
     own.z = (a.row_ptr[3 * r + 1] - own.y) << 8;
-    if (n > 0) own.z |= a.pos[(int64_t)inc[0] * 10 + inc[0] % 10];
+    if (n > 0) {
+      own.z |= a.pos[(int64_t)inc[0] * 10 + inc[0] % 10];
+    } else if (own.z) {
+      // a node of no cell with slots (a pattern of the caller's own): its own column, in the blocks' order
+      const int slot = (a.diag[3 * r] - own.y) / 3;
+      for (int q = 0; q < 3; ++q)
+        if (a.diag[3 * r + q] < 0 || a.diag[3 * r + q] - a.row_ptr[3 * r + q] != 3 * slot + q || slot > 255) *a.fail = 1u;
+      own.z |= slot & 0xff;
+    }
   }
   atomicMax(p.steps + t / kNodes, max(n, 1));  // every group has a step, its last one stores the rows
   p.own[t] = own;
@@ -439,7 +448,8 @@ bool vp2_rows_default(const fe_form_s& f) {
 
 // Builds the plan of an elasticity form bound to a plain pattern, or leaves
 // the form without one (two spaces, restricted dofs, cells with a repeated
-// dof, rows too long for shared memory, no memory for the records).
+// dof, a node of no cell whose diagonal is not in the blocks' order, rows too
+// long for shared memory, no memory for the records).
 void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
   f.nodes_plan.reset();
   if (f.kind != FE_FORM_VP2_ELASTICITY || f.precision != FE_PREC_FP32 || f.V0 != f.V1 || f.V0->excluded ||
@@ -465,6 +475,7 @@ void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
     a.num_cells = C;
     a.num_nodes = nN;
     a.row_ptr = f.sp->row_ptr.p;
+    a.diag = f.sp->diag.p;
     a.dofs = V.dofs.p;
     a.pos = f.pos.p;
     a.inc_ptr = cnt.p;
@@ -528,7 +539,9 @@ void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
       k_nodes_records<<<blocks_for(p.ngroups * kNodes, 128), 128, 0, s>>>(a, p);
       FE_CUDA(cudaGetLastError());
     }
+    FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaStreamSynchronize(s));  // the temporaries are freed on return
+    if (bad) return;
     raise_smem(k_nodes_vp2);
     f.nodes_plan = std::move(P);
   } catch (const Error& e) {
