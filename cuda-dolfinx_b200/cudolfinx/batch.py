@@ -22,17 +22,20 @@ from .context import get_cuda_context
 from .form import CUDAForm
 from .la import CUDAMatrix
 
-# matrix variants worth timing per form kind (all parity-tested)
+# matrix variants worth timing per form kind (all parity-tested).  The row walk
+# stands for itself as "auto": whether it applies depends on the mesh and the
+# pattern, which a size class does not tell, and "auto" goes on with the scatter
+# where it does not
 CANDIDATES = {
-    "P1_STIFFNESS": ("atomic", "block", "tile", "row-walk"),
-    "P2_STIFFNESS": ("atomic", "block", "grouped", "coalesced", "row-walk"),
-    "VP2_ELASTICITY": ("coalesced", "atomic", "atomic-full", "row-walk"),
-    "P3_STIFFNESS": ("coalesced", "atomic", "row-walk"),  # coalesced: FP64 element tensors only (skipped for FP32)
+    "P1_STIFFNESS": ("atomic", "block", "tile", "auto"),
+    "P2_STIFFNESS": ("atomic", "block", "grouped", "coalesced", "auto"),
+    "VP2_ELASTICITY": ("coalesced", "atomic", "atomic-full", "auto"),
+    "P3_STIFFNESS": ("coalesced", "atomic", "auto"),  # coalesced: FP64 element tensors only (skipped for FP32)
 }
-# the row walk is timed from the sizes on where it is the engine's default,
-# for the precision of the element tensors that it takes
-ROW_WALK_CELLS = {"P1_STIFFNESS": 98304, "P2_STIFFNESS": 65536, "P3_STIFFNESS": 0, "VP2_ELASTICITY": 196608}
-ROW_WALK_PRECISION = {"P1_STIFFNESS": "fp64", "P2_STIFFNESS": "fp64", "P3_STIFFNESS": "fp64", "VP2_ELASTICITY": "fp32"}
+# "auto" is timed where the row walk is the engine's default: precision of the
+# element tensors, cells (elsewhere it is one of the others)
+ROW_WALK = {"P1_STIFFNESS": ("fp64", 98304), "P2_STIFFNESS": ("fp64", 65536), "P3_STIFFNESS": ("fp64", 0),
+            "VP2_ELASTICITY": ("fp32", 196608)}
 # FP32 element tensors: variants of one tuple round an entry alike, those of the
 # other tuple differently (5e-9 of the largest entry for P2, 5e-8 for vector P2),
 # so the tuple is chosen by size and only its members are timed: the values do
@@ -43,7 +46,7 @@ ROW_WALK_PRECISION = {"P1_STIFFNESS": "fp64", "P2_STIFFNESS": "fp64", "P3_STIFFN
 # become faster since (n=4 28 us, atomic 58); the line stays, as its values do.
 FP32_VARIANTS = {
     "P2_STIFFNESS": (22000, ("atomic",), ("block", "grouped", "coalesced")),
-    "VP2_ELASTICITY": (38000, ("atomic",), ("coalesced", "row-walk")),
+    "VP2_ELASTICITY": (38000, ("atomic",), ("coalesced", "auto")),
 }
 # launch shapes of the atomic scatter timed per form kind: (cells per CTA,
 # byte maps staged in shared memory)
@@ -91,13 +94,9 @@ class VariantTuner:
         sp = stream.cuda_stream
         best, best_ms, times = None, float("inf"), {}
         trials = []
-        # the row walk takes a field coefficient only when its dofmap is the
-        # mesh's vertex numbering, which the key does not tell: it is timed
-        # for constant and cellwise coefficients
-        field = any(getattr(getattr(c, "function_space", None), "degree", 0) for c in a._spec.coefficients)
+        walk = ROW_WALK.get(a._spec.kind)
         for v in self.candidates(a._spec.kind, a._spec.precision, a._spec.mesh.num_cells):
-            if v == "row-walk" and (field or a._spec.precision != ROW_WALK_PRECISION[a._spec.kind]
-                                    or a._spec.mesh.num_cells < ROW_WALK_CELLS[a._spec.kind]):
+            if v == "auto" and (a._spec.precision != walk[0] or a._spec.mesh.num_cells < walk[1]):
                 continue
             shapes = LAUNCHES.get(a._spec.kind, ((0, 1),)) if v in ("atomic", "atomic-full") else ((0, 1),)
             trials += [(v, shape) for shape in shapes]
