@@ -486,7 +486,9 @@ class FFCxCUDAForm(CUDAForm):
                 dev = self._coef_dev[q]
                 if dev is None or dev.numel() != host.numel():
                     dev = torch.empty(host.numel(), dtype=torch.float64, device=ctx.torch_device)
-                dev.copy_(host, non_blocking=True)  # (waits for the copy unless the host array is page-locked)
+                # the caller may write into the array once the call returns: a page-locked one is waited for (a
+                # pageable one is staged by the copy itself before it returns)
+                dev.copy_(host, non_blocking=not host.is_pinned())
             self._coef_dev[q] = dev
             for h in self._handles:
                 _lib.check(_lib.lib.fe_form_set_coefficient_field(h, q, self._coef_maps[q].handle, dev.data_ptr(),
