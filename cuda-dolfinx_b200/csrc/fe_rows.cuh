@@ -45,7 +45,8 @@ __device__ __forceinline__ RowAt row_at(const RowOut& a, int row) {
 // The warp's 32 row segments (lane l's at acc + l * stride) to their rows.
 // First the segments of rows that a BC touches take their zeros (and a BC row
 // `diagonal` at its own slot, -1: it has none), then all rows are stored, or added
-// with zero == 0.
+// with zero == 0 (by reductions, as the scatter's: another call may add to the
+// same matrix on another stream).
 // A warp takes the `count` rows from `first` on.
 __device__ __forceinline__ void store_rows(const RowOut& a, double* acc, const RowAt& at, int own_slot, int lane,
                                            int first, int count) {
@@ -106,7 +107,7 @@ __device__ __forceinline__ void store_rows(const RowOut& a, double* acc, const R
     for (int s = lane; s < rlen; s += 32) {
       const double v = seg[s];
       if (a.zero) a.values[rlo + s] = v;
-      else a.values[rlo + s] += v;
+      else atomicAdd(a.values + rlo + s, v);
     }
   }
 }

@@ -253,7 +253,7 @@ __device__ __forceinline__ void store_node(const RowOut& a, double* seg, int lo,
     if (f && ((f & 1) || ((__ldg(a.mask + (w >> 5)) >> (w & 31)) & 1u)))
       v = (f & 1) && t - r * len == 3 * own_slot + r ? a.diagonal : 0.0;
     if (a.zero) out[t] = v;
-    else out[t] += v;
+    else atomicAdd(out + t, v);
     seg[t] = 0.0;
   }
 }
