@@ -905,11 +905,11 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
     const bool view = a->sp->parent != nullptr;
     if (view)
       FE_REQUIRE(!(flags & (FE_ASM_DETERMINISTIC | FE_ASM_SORTED_SLOT | FE_ASM_TILE | FE_ASM_ROW_GATHER |
-                            FE_ASM_BLOCK)),
+                            FE_ASM_BLOCK | FE_ASM_ROW_WALK)),
                  "a form bound to a block pattern assembles with the atomic scatter only");
     if (a->ffcx) {
       FE_REQUIRE(!(flags & (FE_ASM_DETERMINISTIC | FE_ASM_SORTED_SLOT | FE_ASM_TILE | FE_ASM_ROW_GATHER |
-                            FE_ASM_BLOCK)),
+                            FE_ASM_BLOCK | FE_ASM_ROW_WALK)),
                  "forms built from FFCx bodies assemble with the atomic scatter only");
       if (zero) launch_zero(values, a->sp->nnz, st);
       ffcx_assemble_matrix(*a, values, bc0, bc1, st);
@@ -918,7 +918,7 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
     }
     if (is_ifacet_kind(a->kind)) {
       FE_REQUIRE(!(flags & (FE_ASM_DETERMINISTIC | FE_ASM_SORTED_SLOT | FE_ASM_TILE | FE_ASM_ROW_GATHER |
-                            FE_ASM_BLOCK)),
+                            FE_ASM_BLOCK | FE_ASM_ROW_WALK)),
                  "interior-facet forms assemble with the atomic scatter only");
       if (zero) launch_zero(values, a->sp->nnz, st);
       assemble_matrix_ifacets(*a, values, bc0, bc1, st);
@@ -927,7 +927,7 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
     }
     if (is_facet_kind(a->kind)) {
       FE_REQUIRE(!(flags & (FE_ASM_DETERMINISTIC | FE_ASM_SORTED_SLOT | FE_ASM_TILE | FE_ASM_ROW_GATHER |
-                            FE_ASM_BLOCK)),
+                            FE_ASM_BLOCK | FE_ASM_ROW_WALK)),
                  "exterior-facet forms assemble with the atomic scatter only");
       FE_REQUIRE(a->V0 == a->V1, "exterior-facet mass forms need the same test and trial dofmap");
       if (zero) launch_zero(values, a->sp->nnz, st);
@@ -983,9 +983,9 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
     // the row walk wherever the form has its plan (built when the pattern was
     // bound) and no other variant is asked for
     if (flags & FE_ASM_ROW_WALK) {
-      if (!a->rows_plan && !view) build_rows_plan(*a, st);
-      if (!a->nodes_plan && !view) build_nodes_plan(*a, st);
-      FE_REQUIRE(!view && (rows_supported(*a, bc0, bc1, st) || vp2_rows_supported(*a, bc0, bc1, st)),
+      if (!a->rows_plan) build_rows_plan(*a, st);
+      if (!a->nodes_plan) build_nodes_plan(*a, st);
+      FE_REQUIRE(rows_supported(*a, bc0, bc1, st) || vp2_rows_supported(*a, bc0, bc1, st),
                  "the row walk supports FP64 P1/P2/P3 stiffness and FP32 vector-P2 elasticity with one space and one "
                  "set of BCs, on conforming cells");
     }
