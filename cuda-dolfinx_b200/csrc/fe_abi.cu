@@ -972,16 +972,17 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
       if (bc0) launch_set_diagonal(*a->sp, *bc0, diagonal, values, st);
       return;
     }
-    // default: the row walk wherever the form has its plan; else the block
-    // variant for P1 meshes above ~1M cells (measured faster on B200 at 12.6M
-    // cells: 0.54 vs 0.73 ms) and the FP64-atomic scatter otherwise (for P2
-    // stiffness and vector P2 with warp-coalesced reductions, below)
+    // default: from the sizes of rows_default / vp2_rows_default on the row walk
+    // where the form has its plan; else the block variant for P1 meshes above
+    // ~1M cells (measured faster on B200 at 12.6M cells: 0.54 vs 0.73 ms) and
+    // the FP64-atomic scatter otherwise (for P2 stiffness and vector P2 with
+    // warp-coalesced reductions, below)
     const bool auto_block = !(flags & FE_ASM_ATOMIC) && !view && a->kind == FE_FORM_P1_STIFFNESS &&
                             a->mesh->num_cells >= (int64_t(1) << 20);
     const bool want_block = (flags & FE_ASM_BLOCK) || auto_block;
     if (flags & FE_ASM_BLOCK) FE_REQUIRE(block_supported(*a), "the block variant supports P1/P2 stiffness only");
-    // the row walk wherever the form has its plan (built when the pattern was
-    // bound) and no other variant is asked for
+    // the row walk where it is asked for, or by default (its plan was built when
+    // the pattern was bound) where no other variant is
     if (flags & FE_ASM_ROW_WALK) {
       if (!a->rows_plan) build_rows_plan(*a, st);
       if (!a->nodes_plan) build_nodes_plan(*a, st);
@@ -989,12 +990,13 @@ int fe_assemble_matrix(fe_form a, double* values, fe_bc bc0, fe_bc bc1, double d
                  "the row walk supports FP64 P1/P2/P3 stiffness and FP32 vector-P2 elasticity with one space and one "
                  "set of BCs, on conforming cells");
     }
+    const bool walk_asked = (flags & FE_ASM_ROW_WALK) != 0;
     if (!(flags & (FE_ASM_ATOMIC | FE_ASM_FULL_SCATTER | FE_ASM_BLOCK | FE_ASM_COALESCED | FE_ASM_GROUPED)) && !view) {
-      if (rows_supported(*a, bc0, bc1, st)) {
+      if ((walk_asked || rows_default(*a)) && rows_supported(*a, bc0, bc1, st)) {
         assemble_matrix_rows(*a, values, bc0, diagonal, zero, st);
         return;
       }
-      if (vp2_rows_supported(*a, bc0, bc1, st)) {
+      if ((walk_asked || vp2_rows_default(*a)) && vp2_rows_supported(*a, bc0, bc1, st)) {
         assemble_matrix_vp2_rows(*a, values, bc0, diagonal, zero, st);
         return;
       }
