@@ -429,71 +429,82 @@ bool valid_identifier(const std::string& s) {
 }
 
 // Moves the tables at the top level of a body -- "[alignas(..)] static const
-// double NAME[..].. = {..};", as FFCx writes them -- to file scope as
-// __constant__ data and returns them; at most `limit` bytes in all (else
-// nothing moves).  In a cell integral every lane reads the same entry at a
-// time, which the constant cache serves in one access; inside a function the
+// double NAME[..].. = {..};", as FFCx writes them, of literals only -- to file
+// scope as __constant__ data and returns them; at most `limit` bytes in all
+// (else nothing moves).  In a cell integral every lane reads the same entry at
+// a time, which the constant cache serves in one access; inside a function the
 // tables are global data, fetched by loads whose latency each use waits for.
+// In the body a reference of the same name takes the table's place, so its
+// scope, its constness and what it hides stay as they were.  A body with
+// preprocessor lines, continued lines or quotes keeps its tables: what this
+// scan reads need not be what is compiled.
+constexpr const char* kTableSpace = "fe_ffcx_tables";
 std::string hoist_tables(std::string& body, size_t limit) {
   std::string rest, tables;
   size_t bytes = 0, at = 0;
   int depth = 0;
-  const std::string key = "static const double ";
+  char before = ';';  // the last character that is neither blank nor in a comment
+  auto blanks = [&](size_t p) { return std::min(body.find_first_not_of(" \t\r\n", p), body.size()); };
   while (at < body.size()) {
-    if (body.compare(at, 2, "//") == 0) {
-      const size_t e = std::min(body.find('\n', at), body.size());
-      rest.append(body, at, e - at);
-      at = e;
-      continue;
-    }
-    if (body.compare(at, 2, "/*") == 0) {
-      const size_t e = body.find("*/", at);
-      const size_t n = e == std::string::npos ? body.size() - at : e + 2 - at;
+    if (body.compare(at, 2, "//") == 0 || body.compare(at, 2, "/*") == 0) {
+      const bool line = body[at + 1] == '/';
+      const size_t e = line ? body.find('\n', at) : body.find("*/", at + 2);
+      const size_t n = e == std::string::npos ? body.size() - at : (line ? e : e + 2) - at;
+      if (line && body.substr(at, n).find('\\') != std::string::npos) return std::string();
       rest.append(body, at, n);
       at += n;
       continue;
     }
-    const bool start = at == 0 || strchr(" \t\n;})", body[at - 1]) != nullptr;
-    if (depth == 0 && start && body.compare(at, key.size(), key) == 0) {
-      // NAME [dims] = { ... } ;
-      size_t q = at + key.size();
-      const size_t semi = body.find(';', q), brack = body.find('[', q), eq = body.find('=', q);
-      if (semi != std::string::npos && brack < eq && eq < semi && body.find_first_of("()", q) > semi) {
+    const char ch = body[at];
+    if (strchr("#\\\"'", ch)) return std::string();
+    if (depth == 0 && (before == ';' || before == '}') && (ch == 'a' || ch == 's')) {
+      // [alignas(N)] static const double NAME [dims] = { ... } ;
+      size_t q = at;
+      if (body.compare(q, 8, "alignas(") == 0) {
+        const size_t digits = body.find_first_not_of("0123456789", q + 8);
+        if (digits != std::string::npos && body[digits] == ')') q = blanks(digits + 1);
+      }
+      const std::string key = "static const double ";
+      const bool found = body.compare(q, key.size(), key) == 0;
+      q += key.size();
+      const size_t semi = found ? body.find(';', q) : std::string::npos;
+      const size_t brack = found ? body.find('[', q) : 0, eq = found ? body.find('=', q) : 0;
+      if (semi != std::string::npos && brack < eq && eq < semi) {
+        const size_t name_end = body.find_last_not_of(" \t\r\n", brack - 1) + 1;
+        const std::string name = name_end > q ? body.substr(q, name_end - q) : std::string();
         size_t count = 1;
-        bool plain = true;
-        for (size_t b = brack; b < eq;) {  // literal dimensions only
+        bool plain = valid_identifier(name);
+        for (size_t b = brack; plain && b < eq;) {  // literal dimensions only
           if (body[b] == '[') {
             char* end = nullptr;
             const unsigned long n = strtoul(body.c_str() + b + 1, &end, 10);
-            plain = plain && n > 0 && n < (1u << 20) && *end == ']';
+            plain = n > 0 && n < (1u << 20) && *end == ']';
             count *= n;
             b = (size_t)(end - body.c_str());
           }
           ++b;
         }
         // literal values only
-        plain = plain && body.find_first_not_of("0123456789.eE+-,{} \t\n=", eq) == semi;
+        plain = plain && body.find_first_not_of("0123456789.eE+-,{} \t\r\n=", eq) == semi;
         if (plain) {
           bytes += 8 * count;
-          // an "alignas(..)" written before it goes along
-          const size_t al = rest.find_last_not_of(" \t\n");
-          if (al != std::string::npos && rest[al] == ')') {
-            const size_t k = rest.rfind("alignas(");
-            if (k != std::string::npos && rest.find(')', k) == al) rest.resize(k);
-          }
           tables += "static __constant__ double " + body.substr(q, semi + 1 - q) + "\n";
+          rest += "const auto& " + name + " = " + kTableSpace + "::" + name + ";";
           at = semi + 1;
+          before = ';';
           continue;
         }
       }
     }
-    if (body[at] == '{') ++depth;
-    if (body[at] == '}') --depth;
-    rest += body[at++];
+    if (ch == '{') ++depth;
+    if (ch == '}') --depth;
+    if (!strchr(" \t\r\n", ch)) before = ch;
+    rest += ch;
+    ++at;
   }
   if (tables.empty() || bytes > limit) return std::string();
   body = rest;
-  return tables;
+  return std::string("namespace ") + kTableSpace + " {\n" + tables + "}\n";
 }
 
 // bilinear forms whose 32 element tensors fit in 48 KB of shared memory and
