@@ -69,7 +69,26 @@ struct FfcxLibrary {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kRegisterTensor = 40;  // entries of an element tensor held in registers
+// Sizes of element tensors, by measurement: from kTileEntries entries on the
+// warp-tile kernel, with the body's tables in constant memory; up to
+// kRegisterTensor its lanes compute the tensor in registers (what spills is
+// rewritten less often than shared memory would be), larger ones in shared
+// memory.  us per call on B200, one thread an entity with its tables where they
+// stand / now (cells of an n^3 cube or its facets):
+//   10x4 P2 x P1 n=37 137 / 93; 8x8 DG1 facets n=20 80..94 / 40..57; 10x10 P2
+//   Robin facets n=40 69 / 56; 10x10 P2 stiffness, 27 points, n=8 53 / 39, n=20
+//   134 / 118, n=37 611 / 559 (647 with the tensor in shared memory); 10x10 P2
+//   stiffness + mass, 8 points, n=20 126 / 68, n=37 539 / 345 (315); 12x12
+//   vector P1 n=20 377 / 191, n=37 2,800 / 895; 20x20 P3 n=20 3,530 / 2,330 and
+//   30x30 vector P2 n=12 3,310 / 1,480 (too large for a tile: the tables alone).
+// Below kTileEntries the tile loses (4x4 P1: Robin facets n=20 9.3 / 13.7,
+// stiffness + mass n=37 85 / 92, Jacobian of exp(u) n=37 227 / 256), and so do
+// the tables as often as not (n=37: 4x4 stiffness 67 / 73, stiffness + mass, 8
+// points, 45 / 53, a 64-point residual 174 / 242): the compiler folds constants
+// that it can see.  Tables of a few numbers make no difference.
+constexpr int kTileEntries = 40;
+constexpr int kRegisterTensor = 100;
+constexpr size_t kTableBytes = 32 * 1024, kFewBytes = 64;
 constexpr int kScalarBlocks = 1024;  // fixed grid of the functional: a fixed summation order
 
 // Kernel argument record.  The generated source declares the same struct
@@ -184,10 +203,9 @@ __device__ __forceinline__ int ffcx_dof1(const FfcxArgs& a, long long e, const i
 // entity after the other, consecutive lanes on consecutive columns of its
 // rows, so that an instruction's reductions share L2 sectors (about two a
 // sector for a P2 cell; 32 lanes on 32 cells' rows have one each).  Bound by
-// the body's own latencies at 8 warps per SM, as many as its tensors in shared
-// memory leave.  P2 stiffness + mass with 8 quadrature points, 304 k cells:
-// 316 us, against 528 us for one thread a cell with the tensor in registers
-// (255 of them, and spills that went to the L2) and the tables in global memory.
+// the body's own latencies at 8 warps per SM, as many as a P2 cell's tensors in
+// shared memory leave; one thread a cell holds the tensor in 255 registers, and
+// its spills go to the L2.
 #define NR (NK0 * BS0)
 #define NC (NK1 * BS1)
 #define ST (NA | 1)
@@ -507,11 +525,12 @@ std::string hoist_tables(std::string& body, size_t limit) {
   return std::string("namespace ") + kTableSpace + " {\n" + tables + "}\n";
 }
 
-// bilinear forms whose 32 element tensors fit in 48 KB of shared memory and
-// whose columns fit in a mask word: the warp-tile kernel (fe_ffcx_mat above)
+// bilinear forms of kTileEntries entries or more whose 32 element tensors fit in
+// 48 KB of shared memory and whose columns fit in a mask word: the warp-tile
+// kernel (fe_ffcx_mat above)
 bool warp_tile(int rank, int rows, int cols) {
-  if (rank != 2 || cols > 32) return false;
   const int na = rows * cols;
+  if (rank != 2 || na < kTileEntries || cols > 32) return false;
   return 32 * ((na | 1) * 8 + rows * 4) <= 48 * 1024;
 }
 
@@ -542,7 +561,8 @@ std::string generate_source(int itype, int rank, int k0, int bs0, int k1, int bs
   replace_all(sk, "@COFF@", off);
   replace_all(sk, "@AREG@", std::to_string(kRegisterTensor));
   std::string code = body;
-  const std::string tables = itype == FE_INTEGRAL_CELL ? hoist_tables(code, 32 * 1024) : std::string();
+  const std::string tables =
+      itype == FE_INTEGRAL_CELL && rank == 2 ? hoist_tables(code, na >= kTileEntries ? kTableBytes : kFewBytes) : std::string();
   std::ostringstream src;
   src << kPreamble << "\n";
   if (!tables.empty()) src << "// the body as given:\n#if 0\n" << body << "\n#endif\n";
@@ -828,7 +848,7 @@ void ffcx_assemble_matrix(fe_form_s& f, double* values, const fe_bc_s* bc0, cons
   const int ns = f.ffcx->integral_type == FE_INTEGRAL_INTERIOR_FACET ? 2 : 1;
   if (warp_tile(2, ns * f.V0->k * f.V0->bs, ns * f.V1->k * f.V1->bs)) {
     void* args[] = {&a};
-    const unsigned grid = (unsigned)std::min<int64_t>((a.num_entities + 31) / 32, 148 * 256);
+    const unsigned grid = (unsigned)std::min<int64_t>((a.num_entities + 31) / 32, f.ctx->num_sms * 256);
     FE_CUDA(cudaLaunchKernel((const void*)f.ffcx->lib->mat, dim3(grid), dim3(32), args, 0, s));
     return;
   }
