@@ -456,14 +456,26 @@ struct CgVectors {
   double* p(int64_t n) const { return z() + (n + 31) / 32 * 32; }
 };
 
-// Up to this many nonzeros -- while a matrix and its vectors stay in the L2 and
-// launches count -- an iteration is the two kernels above; larger matrices keep
-// the five launches (row by row, no pairs: the gather is what counts there).
-// us an iteration on B200, two kernels / five: P2 n=8 (4,913 rows) 15 / 27,
-// n=22 (2.5 M nonzeros) 29 / 33, n=40 (14 M) 95 / 97; P1 n=22 15 / 22, n=64
-// (4 M) 40 / 43, n=110 (20 M) 159 / 155; P3 n=16 (5.5 M) 40 / 41; vector P2
-// n=8 21 / 27, n=20 (17 M) 111 / 73.
-constexpr int64_t kPairNonzeros = 6000000;
+// Whether an iteration is the two kernels above -- while a matrix and its vectors
+// stay in the L2 and launches count -- or the five launches (row by row, no
+// pairs: the gather is what counts there).  The pairs' gather reads 16 bytes a
+// column: that turns the balance sooner where columns are far apart, for short
+// rows from some 300,000 rows on, for the longest rows (three components a
+// node) from 3.5 M nonzeros on; the lines stand a little below.  us an iteration
+// on B200, two kernels / five:
+//   P2 n=8 (4,913 rows) 15 / 27, n=22 (2.5 M nonzeros) 29 / 33, n=29 (5.7 M) 42 /
+//   44, n=40 (14 M) 95 / 97; P3 n=16 (5.5 M) 39.7 / 41; three diagonals, 1.5 M
+//   rows 67 / 71; five, 800,000 rows 44 / 47;
+//   P1 n=22 14 / 22, n=64 (274,625 rows) 39.5 / 41.5, n=66 (300,763) 42.0 / 41.5,
+//   n=70 (357,911) 50 / 46, n=72 55 / 51; seven diagonals, 300,000 rows 30.4 /
+//   33.4, 500,000 rows 41.2 / 39.8;
+//   vector P2 n=8 22 / 26, n=11 (2.9 M nonzeros) 26.9 / 30.5, n=12 (3.8 M) 31.2 /
+//   31.4, n=13 (4.8 M) 33.7 / 33.3, n=14 (5.9 M) 38.5 / 37.5, n=20 (17 M) 111 / 73.
+bool two_kernels(const fe_sparsity_s& A) {
+  const double mean = A.num_rows ? (double)A.nnz / (double)A.num_rows : 0.0;
+  if (mean > 60.0) return A.nnz <= 3200000;
+  return A.nnz <= 6000000 && (mean < 5.5 || mean > 20.0 || A.num_rows <= 280000);
+}
 
 // the launch shapes of both solvers: the row kernels (k_init, k_cg_spmv) wait
 // on dependent loads (row bounds -> columns and values -> gathered entries)
@@ -475,7 +487,7 @@ void cg_begin(const fe_sparsity_s& A, const double* val, const double* b, const 
               const CgVectors& v, unsigned grid, unsigned grid_rows, cudaStream_t s) {
   const int64_t n = A.num_rows;
   FE_CUDA(cudaMemcpyAsync(v.sc, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-  const bool pairs = A.nnz <= kPairNonzeros;
+  const bool pairs = two_kernels(A);
   // (for the pairs z goes through Ap, which is free until the first product; k_init's p is z)
   k_init<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, A.diag.p, b, x, v.r,
                                              pairs ? v.Ap : v.z(), pairs ? v.Ap : v.p(n), v.dinv, v.part);
@@ -502,7 +514,7 @@ template <int SUB>
 void cg_batch(const fe_sparsity_s& A, const double* val, double* x, int count, const CgVectors& v, unsigned grid,
               unsigned grid_rows, cudaStream_t s) {
   const int64_t n = A.num_rows;
-  if (A.nnz > kPairNonzeros) {
+  if (!two_kernels(A)) {
     double *z = v.z(), *p = v.p(n);
     for (int q = 0; q < count; ++q) {
       k_spmv<SUB><<<grid_rows, kThreads, 0, s>>>(n, A.row_ptr.p, A.col.p, val, p, v.Ap, v.part, v.sc);
@@ -547,7 +559,7 @@ void run(const fe_sparsity_s& A, const double* val, const double* b, double* x, 
   cg_begin<SUB>(A, val, b, x, h, v, grid, grid_rows, s);
   // short iterations: a batch is always queued behind the one whose outcome
   // is waited for, so the device does not idle while the host looks at it
-  const bool ahead = A.nnz <= kPairNonzeros;
+  const bool ahead = two_kernels(A);
   const int batch = ahead ? 8 : 16;
   int last = 0;
   for (int k = 0;; ++k) {
