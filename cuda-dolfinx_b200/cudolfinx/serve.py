@@ -90,15 +90,17 @@ def problem_sizes(kind: str, n: int) -> dict:
     return {"cells": cells, "vertices": nv, "rows": rows, "nnz": nnz, "k": k}
 
 
-def slot_bytes(kind: str, n: int) -> int:
+def slot_bytes(kind: str, n: int, precision: str = "fp32") -> int:
     """Device bytes of one slot: CSR values, cell-to-slot map, row-walk plan
     (records of 12, 16 or 20 bytes for a cell's rows, padded, and per row), b, x,
     BC data, solver scratch (6 vectors, an FP32 copy of the values and, for vector P2,
     its block-column index), coefficients."""
     s = problem_sizes(kind, n)
     ncoef = 2 if kind == "vp2" else 1
-    walk = {"p1": 60 * s["cells"] + 16 * s["rows"], "p2": 240 * s["cells"] + 16 * s["rows"],
-            "vp2": 176 * s["cells"] + 8 * s["rows"] if s["cells"] >= 196608 else 0}[kind]
+    # a form binds with a plan from the sizes on, and for the element tensors, where the walk is its default
+    first, tensors, per_cell, per_row = {"p1": (98304, precision, 60, 16), "p2": (65536, "fp64", 240, 16),
+                                         "vp2": (196608, "fp32", 176, 8)}[kind]  # (P1 is always FP64)
+    walk = per_cell * s["cells"] + per_row * s["rows"] if s["cells"] >= first and tensors == precision else 0
     return (8 * s["nnz"] + s["cells"] * s["k"] * s["k"] + walk + 8 * 2 * s["rows"] + 9 * s["rows"] + 8 * 6 * s["rows"]
             + 4 * s["nnz"] + (s["nnz"] // 9 * 4 + s["rows"] // 3 * 4 if kind == "vp2" else 0)
             + 8 * ncoef * s["cells"])
@@ -352,7 +354,7 @@ class Server:
         import torch
         with torch.cuda.stream(self._streams[0]):
             for key in keys:
-                nb, sb = slot_bytes(*key), shared_bytes(*key)
+                nb, sb = slot_bytes(*key, self.precision), shared_bytes(*key)
                 st, _ = self.ledger.reserve(key, nb, sb)
                 if st != "new":
                     continue
@@ -382,7 +384,7 @@ class Server:
                     while True:
                         if pending:
                             req = pending[0]
-                            nb, sb = slot_bytes(*req.key), shared_bytes(*req.key)
+                            nb, sb = slot_bytes(*req.key, self.precision), shared_bytes(*req.key)
                             if self.plain:
                                 status, slot = self.ledger.reserve(("plain",) + req.key, nb, sb)
                             else:
