@@ -113,18 +113,29 @@ __global__ void k_rows_fill(const PlanArgs a, int32_t* __restrict__ cursor) {
 }
 
 // sort key of a row: kind, window of 1024 rows (so that a warp's rows stay
-// close in memory), number of cells
+// close in memory), number of cells; per kind its rows and the longest of them
+// (totals[kind], totals[3 + kind])
 __global__ void k_rows_keys(const PlanArgs a, const int32_t* __restrict__ cnt, const unsigned* __restrict__ kmask,
-                            uint32_t* __restrict__ key, int32_t* __restrict__ row, int* __restrict__ kinds) {
+                            uint32_t* __restrict__ key, int32_t* __restrict__ row, int* __restrict__ totals) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= a.num_rows) return;
-  const unsigned m = kmask[r];
-  if (m & (m - 1)) *a.fail = 1u;  // a node that is a vertex here and an edge node there
-  const int kind = m & 4u ? KIND_F : (m & 2u ? KIND_E : KIND_V);
-  const int n = min(cnt[r], 255);
-  key[r] = ((uint32_t)kind << 30) | ((uint32_t)(r >> 10) << 8) | (uint32_t)n;
-  row[r] = (int32_t)r;
-  atomicAdd(kinds + kind, 1);
+  int kind = -1, len = 0;
+  if (r < a.num_rows) {
+    const unsigned m = kmask[r];
+    if (m & (m - 1)) *a.fail = 1u;  // a node that is a vertex here and an edge node there
+    kind = m & 4u ? KIND_F : (m & 2u ? KIND_E : KIND_V);
+    len = a.row_ptr[r + 1] - a.row_ptr[r];
+    const int n = min(cnt[r], 255);
+    key[r] = ((uint32_t)kind << 30) | ((uint32_t)(r >> 10) << 8) | (uint32_t)n;
+    row[r] = (int32_t)r;
+  }
+  for (int k = 0; k < 3; ++k) {
+    const unsigned here = __ballot_sync(kAll, kind == k);
+    if (!here) continue;
+    const int most = __reduce_max_sync(kAll, kind == k ? len : 0);
+    if ((threadIdx.x & 31) != 0) continue;
+    atomicAdd(totals + k, __popc(here));
+    if (most > totals[3 + k]) atomicMax(totals + 3 + k, most);
+  }
 }
 
 // the cell's vertices in the row's order: positions p[0..3]
@@ -1382,20 +1393,31 @@ void build_rows_plan(fe_form_s& f, cudaStream_t s) {
       mesh.num_nodes > kStripVertex ||
       capturing(s))
     return;
-  int longest = 0;
-  for (int64_t r = 0; r < nR; ++r)
-    longest = std::max(longest, f.sp->host_row_ptr[r + 1] - f.sp->host_row_ptr[r]);
-  if (longest > 256) return;
   try {
     auto P = std::make_unique<fe_form_s::RowsPlan>();
-    DevBuf<int32_t> cnt(nR + 1), cursor(nR + 1), inc((size_t)C * V.k), row(nR), row_sorted(nR);
-    DevBuf<unsigned> kmask(nR), fail(1);
-    DevBuf<uint32_t> key(nR), key_sorted(nR);
-    DevBuf<int> kinds(3);
-    FE_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes(), s));
-    FE_CUDA(cudaMemsetAsync(kmask.p, 0, kmask.bytes(), s));
-    FE_CUDA(cudaMemsetAsync(fail.p, 0, fail.bytes(), s));
-    FE_CUDA(cudaMemsetAsync(kinds.p, 0, kinds.bytes(), s));
+    // the temporaries in one allocation (a large one takes 0.3 ms, and as long to give back)
+    size_t tb = 0;
+    FE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr,
+                                            (int32_t*)nullptr, (int)nR, 0, 32, s));
+    DevBuf<int32_t> work((tb + 3) / 4 + (size_t)C * V.k + 7 * (size_t)(nR + 1) + 8);
+    int32_t* next = work.p;
+    auto take = [&](size_t n) {
+      int32_t* q = next;
+      next += n;
+      return q;
+    };
+    void* tmp = take((tb + 3) / 4);
+    int32_t* cnt = take(nR + 1);
+    unsigned* kmask = reinterpret_cast<unsigned*>(take(nR + 1));
+    int* totals = take(6);
+    unsigned* fail = reinterpret_cast<unsigned*>(take(1));
+    FE_CUDA(cudaMemsetAsync(cnt, 0, (2 * (size_t)(nR + 1) + 7) * sizeof(int32_t), s));
+    int32_t* cursor = take(nR + 1);
+    int32_t* row = take(nR);
+    int32_t* row_sorted = take(nR);
+    uint32_t* key = reinterpret_cast<uint32_t*>(take(nR));
+    uint32_t* key_sorted = reinterpret_cast<uint32_t*>(take(nR));
+    int32_t* inc = take((size_t)C * V.k);
     PlanArgs a{};
     a.num_cells = C;
     a.num_rows = nR;
@@ -1406,27 +1428,29 @@ void build_rows_plan(fe_form_s& f, cudaStream_t s) {
     a.pos = f.pos.p;
     a.row_ptr = f.sp->row_ptr.p;
     a.diag = f.sp->diag.p;
-    a.inc_ptr = cnt.p;
-    a.inc = inc.p;
-    a.fail = fail.p;
-    k_rows_count<<<blocks_for(C, 128), 128, 0, s>>>(a, cnt.p, kmask.p);
+    a.inc_ptr = cnt;
+    a.inc = inc;
+    a.fail = fail;
+    k_rows_count<<<blocks_for(C, 128), 128, 0, s>>>(a, cnt, kmask);
     FE_CUDA(cudaGetLastError());
-    k_rows_keys<<<blocks_for(nR, 256), 256, 0, s>>>(a, cnt.p, kmask.p, key.p, row.p, kinds.p);
+    k_rows_keys<<<blocks_for(nR, 256), 256, 0, s>>>(a, cnt, kmask, key, row, totals);
     FE_CUDA(cudaGetLastError());
-    exclusive_scan(cnt.p, nR + 1, s);
-    int hk[3];
-    unsigned bad = 0;
-    FE_CUDA(cudaMemcpyAsync(hk, kinds.p, sizeof(hk), cudaMemcpyDeviceToHost, s));
-    FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
-    FE_CUDA(cudaMemcpyAsync(cursor.p, cnt.p, cursor.bytes(), cudaMemcpyDeviceToDevice, s));
+    exclusive_scan(cnt, nR + 1, s);
+    int h[7];  // rows of each kind, their longest, the mark of a failed plan
+    FE_CUDA(cudaMemcpyAsync(h, totals, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FE_CUDA(cudaMemcpyAsync(cursor, cnt, (size_t)(nR + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
     FE_CUDA(cudaStreamSynchronize(s));
-    if (bad) return;
-    k_rows_fill<<<blocks_for(C * V.k, 256), 256, 0, s>>>(a, cursor.p);
+    const int *hk = h, *longest = h + 3;
+    if (h[6] || std::max({longest[0], longest[1], longest[2]}) > 256) return;
+    // segments as long as the longest row of the kind; at least four warps per
+    // SM, or the scatter is the better one
+    for (int kind = 0; kind < 3; ++kind) {
+      P->part[kind].stride = odd_at_least(longest[kind]);
+      if (segment_bytes(P->part[kind].stride) + kSmemCta > kSmemSm / 4) return;
+    }
+    k_rows_fill<<<blocks_for(C * V.k, 256), 256, 0, s>>>(a, cursor);
     FE_CUDA(cudaGetLastError());
-    size_t tb = 0;
-    FE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key_sorted.p, row.p, row_sorted.p, (int)nR, 0, 32, s));
-    DevBuf<unsigned char> tmp(std::max<size_t>(1, tb));
-    FE_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key_sorted.p, row.p, row_sorted.p, (int)nR, 0, 32, s));
+    FE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key_sorted, row, row_sorted, (int)nR, 0, 32, s));
     int64_t first = 0;
     for (int kind = 0; kind < 3; ++kind) {
       PartArgs p{};
@@ -1440,30 +1464,18 @@ void build_rows_plan(fe_form_s& f, cudaStream_t s) {
       p.parts = 1;
       if (kind == KIND_V) p.parts = p.ngroups <= 2 * f.ctx->num_sms ? 4 : (p.ngroups <= 10 * f.ctx->num_sms ? 2 : 1);
       if (p.nrows == 0) continue;
-      build_part(a, p, P->part[kind], row_sorted.p + first, s);
+      build_part(a, p, P->part[kind], row_sorted + first, s);
       first += p.nrows;
     }
     P->x4.alloc((size_t)std::max<int64_t>(1, mesh.num_nodes));
     k_rows_pad_x<<<blocks_for(mesh.num_nodes, 256), 256, 0, s>>>(mesh.x.p, mesh.num_nodes, P->x4.p);
     FE_CUDA(cudaGetLastError());
-    FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
+    unsigned bad = 0;
+    FE_CUDA(cudaMemcpyAsync(&bad, fail, sizeof(bad), cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaStreamSynchronize(s));  // the temporaries are freed on return
     if (bad) return;
-    // segments as long as the longest row of the kind
-    std::vector<int32_t> order((size_t)nR);
-    FE_CUDA(cudaMemcpy(order.data(), row_sorted.p, order.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
-    int64_t at = 0;
-    for (int kind = 0; kind < 3; ++kind) {
-      int len = 0;
-      for (const int64_t end = at + hk[kind]; at < end; ++at)
-        len = std::max(len, f.sp->host_row_ptr[order[at] + 1] - f.sp->host_row_ptr[order[at]]);
-      P->part[kind].stride = odd_at_least(len);
-    }
-    // at least four warps per SM, or the scatter is the better one
-    for (auto& part : P->part) {
-      if (segment_bytes(part.stride) + kSmemCta > kSmemSm / 4) return;
+    for (auto& part : P->part)
       while (part.parts > 1 && part.parts * segment_bytes(part.stride) + kSmemCta > kSmemSm) part.parts /= 2;
-    }
     if (deg == 1) raise_all<1>();
     else if (deg == 2) raise_all<2>();
     else raise_p3();

@@ -85,14 +85,28 @@ __global__ void k_nodes_fill(const VPlanArgs a, int32_t* __restrict__ cursor) {
   a.inc[atomicAdd(cursor + a.dofs[t], 1)] = (int32_t)t;
 }
 
-// sort key: edge nodes after vertices, window of 1024 nodes, number of cells
+// sort key: edge nodes after vertices, window of 1024 nodes, number of cells;
+// totals: the vertices, then the longest row of the vertices and of the others
 __global__ void k_nodes_keys(const VPlanArgs a, const int32_t* __restrict__ cnt, const uint8_t* __restrict__ vertex,
-                             uint32_t* __restrict__ key, int32_t* __restrict__ node, int* __restrict__ vertices) {
+                             uint32_t* __restrict__ key, int32_t* __restrict__ node, int* __restrict__ totals) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= a.num_nodes) return;
-  key[r] = (vertex[r] ? 0u : 1u << 30) | ((uint32_t)(r >> 10) << 8) | (uint32_t)min(cnt[r], 255);
-  node[r] = (int32_t)r;
-  if (vertex[r]) atomicAdd(vertices, 1);
+  int kind = -1, len = 0;
+  if (r < a.num_nodes) {
+    kind = vertex[r] ? 0 : 1;
+    const int32_t* p = a.row_ptr + 3 * r;
+    len = p[1] - p[0];
+    if (p[2] - p[1] != len || p[3] - p[2] != len) *a.fail = 1u;
+    key[r] = ((uint32_t)kind << 30) | ((uint32_t)(r >> 10) << 8) | (uint32_t)min(cnt[r], 255);
+    node[r] = (int32_t)r;
+  }
+  for (int k = 0; k < 2; ++k) {
+    const unsigned here = __ballot_sync(kAll, kind == k);
+    if (!here) continue;
+    const int most = __reduce_max_sync(kAll, kind == k ? len : 0);
+    if ((threadIdx.x & 31) != 0) continue;
+    if (k == 0) atomicAdd(totals, __popc(here));
+    if (most > totals[1 + k]) atomicMax(totals + 1 + k, most);
+  }
 }
 
 struct VPartArgs {
@@ -462,15 +476,29 @@ void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
     return;
   try {
     auto P = std::make_unique<fe_form_s::NodesPlan>();
-    DevBuf<int32_t> cnt(nN + 1), cursor(nN + 1), inc((size_t)C * 10), node(nN), sorted(nN);
-    DevBuf<uint8_t> vertex(nN);
-    DevBuf<uint32_t> key(nN), key_sorted(nN);
-    DevBuf<unsigned> fail(1);
-    DevBuf<int> vertices(1);
-    FE_CUDA(cudaMemsetAsync(cnt.p, 0, cnt.bytes(), s));
-    FE_CUDA(cudaMemsetAsync(vertex.p, 0, vertex.bytes(), s));
-    FE_CUDA(cudaMemsetAsync(fail.p, 0, fail.bytes(), s));
-    FE_CUDA(cudaMemsetAsync(vertices.p, 0, vertices.bytes(), s));
+    // the temporaries in one allocation (a large one takes 0.3 ms, and as long to give back)
+    size_t tb = 0;
+    FE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr,
+                                            (int32_t*)nullptr, (int)nN, 0, 31, s));
+    DevBuf<int32_t> work((tb + 3) / 4 + (size_t)C * 10 + 7 * (size_t)(nN + 1) + 4);
+    int32_t* next = work.p;
+    auto take = [&](size_t n) {
+      int32_t* q = next;
+      next += n;
+      return q;
+    };
+    void* tmp = take((tb + 3) / 4);
+    int32_t* cnt = take(nN + 1);
+    uint8_t* vertex = reinterpret_cast<uint8_t*>(take(nN / 4 + 1));
+    int* totals = take(3);
+    unsigned* fail = reinterpret_cast<unsigned*>(take(1));
+    FE_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(next - cnt) * sizeof(int32_t), s));
+    int32_t* cursor = take(nN + 1);
+    int32_t* node = take(nN);
+    int32_t* sorted = take(nN);
+    uint32_t* key = reinterpret_cast<uint32_t*>(take(nN));
+    uint32_t* key_sorted = reinterpret_cast<uint32_t*>(take(nN));
+    int32_t* inc = take((size_t)C * 10);
     VPlanArgs a{};
     a.num_cells = C;
     a.num_nodes = nN;
@@ -478,44 +506,27 @@ void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
     a.diag = f.sp->diag.p;
     a.dofs = V.dofs.p;
     a.pos = f.pos.p;
-    a.inc_ptr = cnt.p;
-    a.inc = inc.p;
-    a.fail = fail.p;
-    k_nodes_count<<<blocks_for(C, 128), 128, 0, s>>>(a, cnt.p, vertex.p);
+    a.inc_ptr = cnt;
+    a.inc = inc;
+    a.fail = fail;
+    k_nodes_count<<<blocks_for(C, 128), 128, 0, s>>>(a, cnt, vertex);
     FE_CUDA(cudaGetLastError());
-    k_nodes_keys<<<blocks_for(nN, 256), 256, 0, s>>>(a, cnt.p, vertex.p, key.p, node.p, vertices.p);
+    k_nodes_keys<<<blocks_for(nN, 256), 256, 0, s>>>(a, cnt, vertex, key, node, totals);
     FE_CUDA(cudaGetLastError());
-    exclusive_scan(cnt.p, nN + 1, s);
-    unsigned bad = 0;
-    int nv = 0;
-    FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
-    FE_CUDA(cudaMemcpyAsync(&nv, vertices.p, sizeof(nv), cudaMemcpyDeviceToHost, s));
-    FE_CUDA(cudaMemcpyAsync(cursor.p, cnt.p, cursor.bytes(), cudaMemcpyDeviceToDevice, s));
+    exclusive_scan(cnt, nN + 1, s);
+    int h[4];  // the vertices, the longest rows, the mark of a failed plan
+    FE_CUDA(cudaMemcpyAsync(h, totals, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FE_CUDA(cudaMemcpyAsync(cursor, cnt, (size_t)(nN + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
     FE_CUDA(cudaStreamSynchronize(s));
-    if (bad) return;
-    k_nodes_fill<<<blocks_for(C * 10, 256), 256, 0, s>>>(a, cursor.p);
+    if (h[3]) return;
+    k_nodes_fill<<<blocks_for(C * 10, 256), 256, 0, s>>>(a, cursor);
     FE_CUDA(cudaGetLastError());
-    size_t tb = 0;
-    FE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.p, key_sorted.p, node.p, sorted.p, (int)nN, 0, 31, s));
-    DevBuf<unsigned char> tmp(std::max<size_t>(1, tb));
-    FE_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.p, key_sorted.p, node.p, sorted.p, (int)nN, 0, 31, s));
-    std::vector<int32_t> order((size_t)nN);
-    FE_CUDA(cudaMemcpyAsync(order.data(), sorted.p, order.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    FE_CUDA(cudaStreamSynchronize(s));
+    FE_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tb, key, key_sorted, node, sorted, (int)nN, 0, 31, s));
     for (int kind = 0; kind < 2; ++kind) {
       auto& part = P->part[kind];
-      const int64_t first = kind ? nv : 0, count = kind ? nN - nv : nv;
+      const int64_t first = kind ? h[0] : 0, count = kind ? nN - h[0] : h[0];
       if (!count) continue;
-      int longest = 0;
-      for (int64_t t = first; t < first + count; ++t) {
-        const int64_t r = 3 * (int64_t)order[t];
-        const int len = f.sp->host_row_ptr[r + 1] - f.sp->host_row_ptr[r];
-        if (f.sp->host_row_ptr[r + 2] - f.sp->host_row_ptr[r + 1] != len ||
-            f.sp->host_row_ptr[r + 3] - f.sp->host_row_ptr[r + 2] != len)
-          return;
-        longest = std::max(longest, len);
-      }
-      part.stride = (3 * std::max(longest, 3) + 2) & ~1;  // and one for the phase of its range
+      part.stride = (3 * std::max(h[1 + kind], 3) + 2) & ~1;  // and one for the phase of its range
       // (at least two groups per SM)
       if (nodes_smem(part.stride) + kSmemCta > kSmemSm / 2) return;
       part.ngroups = (count + kNodes - 1) / kNodes;
@@ -525,7 +536,7 @@ void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
       VPartArgs p{};
       p.count = count;
       p.ngroups = part.ngroups;
-      p.nodes = sorted.p + first;
+      p.nodes = sorted + first;
       p.own = part.own.p;
       p.steps = part.steps.p;
       k_nodes_head<<<blocks_for(p.ngroups * kNodes, 128), 128, 0, s>>>(a, p);
@@ -539,7 +550,8 @@ void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
       k_nodes_records<<<blocks_for(p.ngroups * kNodes, 128), 128, 0, s>>>(a, p);
       FE_CUDA(cudaGetLastError());
     }
-    FE_CUDA(cudaMemcpyAsync(&bad, fail.p, sizeof(bad), cudaMemcpyDeviceToHost, s));
+    unsigned bad = 0;
+    FE_CUDA(cudaMemcpyAsync(&bad, fail, sizeof(bad), cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaStreamSynchronize(s));  // the temporaries are freed on return
     if (bad) return;
     raise_smem(k_nodes_vp2);
