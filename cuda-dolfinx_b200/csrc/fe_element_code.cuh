@@ -1726,6 +1726,7 @@ __device__ __forceinline__ void p2_mass_p1coef(const T* cq, Emit&& emit) {
   emit(9, 9, (fma(cq[2], T(0x1.a01a01a01a01ap-10), cq[0] * T(0x1.3813813813814p-8)) + fma(cq[3], T(0x1.a01a01a01a01ap-10), cq[1] * T(0x1.3813813813814p-8))));
 }
 
+#ifdef FE_P3_ROW_TABLES
 // P3 stiffness row of vertex a: g[q] = k |det J| times the products of the gradients
 // ab, ac, ad, bc, bd, cd; emit(column, value), columns a, b, c, d, ab ba ac ca ad da bc cb bd db cd dc (xy: on edge xy near x), abc abd acd bcd.
 __constant__ double kP3RowV[9] = {
@@ -1816,6 +1817,8 @@ __device__ __forceinline__ void p3_row_f(const double* g, Emit&& emit) {
   emit(18, g[1] * kP3RowF[9] + g[4] * kP3RowF[10]);
   emit(19, g[2] * kP3RowF[10] + g[3] * kP3RowF[9]);
 }
+
+#endif  // FE_P3_ROW_TABLES
 
 #ifdef FE_FACET_TABLES
 // cell-local dofs on each facet (P1)

@@ -34,6 +34,7 @@
 #include <cub/cub.cuh>
 #include <memory>
 
+#define FE_P3_ROW_TABLES
 #include "fe_element_code.cuh"
 #include "fe_internal.h"
 #include "fe_rows.cuh"

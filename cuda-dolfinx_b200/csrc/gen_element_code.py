@@ -431,7 +431,11 @@ def p3_row_tables() -> str:
     the node is vertex a, the node of edge ab near a, or the node of face abc.
     With g_x the gradients of the barycentric coordinates, an entry is
     sum_xy c_xy g_x.g_y, c_xy = int d_x phi_i d_y phi_j over the barycentric
-    derivatives; g_x.g_x = -sum_{y != x} g_x.g_y leaves the six products x < y."""
+    derivatives; g_x.g_x = -sum_{y != x} g_x.g_y leaves the six products x < y.
+    Compiled only where FE_P3_ROW_TABLES is defined: a constant table is in the
+    constant bank of every kernel of a unit that has it, and each launch pays
+    for the bank (a graph of 14 P1 / P2 meshes, n <= 10, on B200: 57 us a replay,
+    60.5 with these 296 bytes in the scatter's unit)."""
     lam = [tuple(1 if q == v else 0 for q in range(4)) for v in range(4)]
 
     def mul(p, q):
@@ -497,7 +501,7 @@ def p3_row_tables() -> str:
         "f": "a, b, c, ab ba ac ca bc cb, abc, d, ad da bd db cd dc, abd, acd, bcd",
     }
     pairs = [(a, b), (a, c), (a, d), (b, c), (b, d), (c, d)]
-    out = []
+    out = ["#ifdef FE_P3_ROW_TABLES\n"]
     for kind in ("v", "e", "f"):
         out.append(f"// P3 stiffness row of {what[kind]}: g[q] = k |det J| times the products of the gradients\n"
                    f"// ab, ac, ad, bc, bd, cd; emit(column, value), columns {order[kind]}.\n")
@@ -526,6 +530,7 @@ def p3_row_tables() -> str:
         out.append(f"__device__ __forceinline__ void p3_row_{kind}(const double* g, Emit&& emit) {{\n")
         out += body
         out.append("}\n\n")
+    out.append("#endif  // FE_P3_ROW_TABLES\n\n")
     return "".join(out)
 
 
