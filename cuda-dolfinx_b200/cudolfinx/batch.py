@@ -95,8 +95,11 @@ class VariantTuner:
         best, best_ms, times = None, float("inf"), {}
         trials = []
         walk = ROW_WALK.get(a._spec.kind)
+        # whether the walk takes a field coefficient depends on its dofmap, which the key does not tell: it is
+        # timed for constant and cellwise ones
+        field = any(getattr(getattr(c, "function_space", None), "degree", 0) for c in a._spec.coefficients)
         for v in self.candidates(a._spec.kind, a._spec.precision, a._spec.mesh.num_cells):
-            if v == "auto" and (a._spec.precision != walk[0] or a._spec.mesh.num_cells < walk[1]):
+            if v == "auto" and (field or a._spec.precision != walk[0] or a._spec.mesh.num_cells < walk[1]):
                 continue
             shapes = LAUNCHES.get(a._spec.kind, ((0, 1),)) if v in ("atomic", "atomic-full") else ((0, 1),)
             trials += [(v, shape) for shape in shapes]
