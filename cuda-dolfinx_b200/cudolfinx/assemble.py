@@ -153,8 +153,9 @@ class CUDAAssembler:
         "row-walk" (FP64 P1/P2/P3 stiffness, FP32 vector-P2 elasticity: the
         cells around a row's node are added up by the row's own thread or warp;
         bitwise reproducible; not offered for two different
-        spaces or BCs, block patterns, dofs shared between several vertices
-        or overlapping cells),
+        spaces or BCs, block patterns, dofs shared between several vertices,
+        overlapping cells, neighbours that do not share the dofs of a common
+        face, FFCx and facet forms),
         "deterministic" (bitwise reproducible: ordered tile gather for P1/P2,
         sorted-slot otherwise), "atomic" (FP64-atomic scatter, one thread's
         reductions per cell), "coalesced" (P2, vector P2, FP64 P3: a warp's
