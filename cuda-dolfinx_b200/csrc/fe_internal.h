@@ -313,11 +313,12 @@ struct fe_form_s::RowsPlan {
     bool gaps = false;                // some rows have slots that no cell adds to
     fe::DevBuf<int4> own;             // [groups*32] row (-1: none), its vertices, the slots of its own columns
     fe::DevBuf<int32_t> steps;        // [groups+1] prefix sums of the groups' longest walks
-    fe::DevBuf<uint4> rec;            // records: vertices with marks, slot bytes
-    fe::DevBuf<uint4> rec2;           // P3: the rest of the records
     fe::DevBuf<int4> own2;            // P3 face rows: the slots of their own columns
-    fe::DevBuf<uint2> rec1;           // P1 records
-    fe::DevBuf<int32_t> cell;         // cell of each record
+    fe::DevBuf<unsigned char> mem;    // the records, in this:
+    uint4* rec = nullptr;             // vertices with marks, slot bytes
+    uint4* rec2 = nullptr;            // P3: the rest of the records
+    uint2* rec1 = nullptr;            // P1 records
+    int32_t* cell = nullptr;          // cell of each record
   };
   Part part[3];
   fe::DevBuf<double4> x4;             // vertex coordinates, 32 bytes apart
@@ -573,6 +574,9 @@ void reset_batch_plan(fe_form_s& f);
 void assemble_matrix_batch(fe_form_s& f, int num_instances, const double* const* coefficients,
                            double* const* values, const fe_bc_s* bc0, const fe_bc_s* bc1, double diagonal,
                            bool zero, cudaStream_t s);
+
+// the context's pool of stream-ordered scratch (fe_pcg.cu)
+cudaMemPool_t scratch_pool(fe_context_s& ctx);
 
 // row-walk assembly (fe_rows.cu): where it is the default (rows_default) the
 // plan is built with the slot map; build_rows_plan leaves none where the walk

@@ -361,10 +361,10 @@ __global__ void __launch_bounds__(kThreads) k_update_p(int64_t n, const double* 
     p[i] = z[i] + beta * p[i];
 }
 
-// cudaMallocAsync'd buffers freed with cudaFreeAsync on the same stream when
-// the scope ends, normally or by an exception.
+}  // namespace
+
 cudaMemPool_t scratch_pool(fe_context_s& ctx) {
-  static std::mutex m;  // solver calls on several host threads share the context
+  static std::mutex m;  // calls on several host threads share the context
   std::lock_guard<std::mutex> lock(m);
   if (!ctx.scratch_pool) {
     cudaMemPoolProps props{};
@@ -382,6 +382,9 @@ cudaMemPool_t scratch_pool(fe_context_s& ctx) {
   return ctx.scratch_pool;
 }
 
+namespace {
+// cudaMallocAsync'd buffers freed with cudaFreeAsync on the same stream when
+// the scope ends, normally or by an exception.
 struct StreamScratch {
   cudaStream_t s;
   cudaMemPool_t pool;

@@ -212,6 +212,45 @@ __device__ __forceinline__ void load_cell(const PlanArgs& a, int32_t t, int64_t&
   g[3] = v.w;
 }
 
+// The triangles opposite a vertex in its cells, and for each of their edges
+// (opposite corner e) the other triangle that has it.
+constexpr int kNoTriangle = 255;
+struct Star {
+  int n;
+  int tv[kMaxStar][3];           // mesh vertices
+  uint8_t nb[kMaxStar][3];
+  bool simple;                   // no edge is in three triangles, no triangle there twice
+};
+
+__device__ void load_star(const PlanArgs& a, const int32_t* inc, int n, Star& S) {
+  S.n = n;
+  S.simple = true;
+  for (int t = 0; t < n; ++t) {
+    int64_t c;
+    int i, g[4];
+    load_cell(a, inc[t], c, i, g);
+    int q = 0;
+    for (int v = 0; v < 4; ++v)
+      if (v != i) S.tv[t][q++] = g[v];
+    const int x = S.tv[t][0], y = S.tv[t][1], z = S.tv[t][2];
+    if (x == y || x == z || y == z) S.simple = false;
+    for (int e = 0; e < 3; ++e) S.nb[t][e] = kNoTriangle;
+    for (int o = 0; o < t; ++o) {
+      // corners that the other triangle does not have
+      const int ox = S.tv[o][0], oy = S.tv[o][1], oz = S.tv[o][2];
+      const int miss = (x != ox && x != oy && x != oz ? 1 : 0) | (y != ox && y != oy && y != oz ? 2 : 0) |
+                       (z != ox && z != oy && z != oz ? 4 : 0);
+      if (miss == 0) S.simple = false;
+      if (miss != 1 && miss != 2 && miss != 4) continue;
+      const int e = miss >> 1;  // 0, 1, 2
+      const int f = ox != x && ox != y && ox != z ? 0 : (oy != x && oy != y && oy != z ? 1 : 2);
+      if (S.nb[t][e] != kNoTriangle || S.nb[o][f] != kNoTriangle) S.simple = false;
+      S.nb[t][e] = (uint8_t)o;
+      S.nb[o][f] = (uint8_t)t;
+    }
+  }
+}
+
 // The cells of a vertex row as strips of the triangles opposite the vertex,
 // cut into `parts` of nearly as many cells: emit(part, cell entry, its three
 // other vertices, flags) for each step, cell entry -1 for the two steps that
@@ -219,18 +258,11 @@ __device__ __forceinline__ void load_cell(const PlanArgs& a, int32_t t, int64_t&
 // first strip begins: its triangle, which of its vertices is left first, and
 // which way it goes at a tie.
 template <typename Emit>
-__device__ int walk_star(const PlanArgs& a, const int32_t* inc, int n, int parts, int code, Emit&& emit) {
-  int tv[kMaxStar][3];           // mesh vertices opposite the row's
+__device__ int walk_star(const Star& S, int parts, int code, Emit&& emit) {
+  const int n = S.n;
+  const int(*tv)[3] = S.tv;
   uint32_t used[kMaxStar / 32];
   for (int q = 0; q < kMaxStar / 32; ++q) used[q] = 0u;
-  for (int t = 0; t < n; ++t) {
-    int64_t c;
-    int i, g[4];
-    load_cell(a, inc[t], c, i, g);
-    int q = 0;
-    for (int v = 0; v < 4; ++v)
-      if (v != i) tv[t][q++] = g[v];
-  }
   auto is_used = [&](int t) { return (used[t >> 5] >> (t & 31)) & 1u; };
   auto has = [&](int t, int v) { return tv[t][0] == v || tv[t][1] == v || tv[t][2] == v; };
   // the free triangle with vertices u and v, -1 if there is none
@@ -243,6 +275,14 @@ __device__ int walk_star(const PlanArgs& a, const int32_t* inc, int n, int parts
     for (int q = 0; q < 3; ++q)
       if (tv[t][q] != u && tv[t][q] != v) return tv[t][q];
     return u;
+  };
+  // across the edge of t opposite its corner `off`, whose ends are u and v: the
+  // first free triangle but t, -1 if there is none
+  auto across = [&](int t, int off, int u, int v) -> int {
+    if (!S.simple) return find(u, v);
+    const int e = tv[t][0] == off ? 0 : (tv[t][1] == off ? 1 : 2);
+    const int o = S.nb[t][e];
+    return o != kNoTriangle && !is_used(o) ? o : -1;
   };
   int steps = 0, longest = 0, left = n, first = 0, part = 0, done = 0;
   auto next_part = [&]() {  // after `done` cells
@@ -268,12 +308,12 @@ __device__ int walk_star(const PlanArgs& a, const int32_t* inc, int n, int parts
       q = tv[t][(turn + 1) % 3];
       r = tv[t][(turn + 2) % 3];
       begun = true;
-    } else if (find(q, r) < 0) {
-      if (find(p, r) >= 0) {
+    } else if (across(t, p, q, r) < 0) {
+      if (across(t, q, p, r) >= 0) {
         const int w = p;
         p = q;
         q = w;
-      } else if (find(p, q) >= 0) {
+      } else if (across(t, r, p, q) >= 0) {
         const int w = p;
         p = r;
         r = w;
@@ -283,7 +323,7 @@ __device__ int walk_star(const PlanArgs& a, const int32_t* inc, int n, int parts
     emit(part, -1, q, 0, 0, kStripLoad);
     steps += 2;
     while (true) {
-      const int t1 = find(q, r), t2 = find(p, r);
+      const int t1 = across(t, p, q, r), t2 = across(t, q, p, r);
       int next = t1;
       bool keep = false;
       if (t2 >= 0) {
@@ -293,7 +333,11 @@ __device__ int walk_star(const PlanArgs& a, const int32_t* inc, int n, int parts
           // towards the triangle with fewer free neighbours
           auto degree = [&](int x, int u, int v) {
             const int w = third(x, u, v);
-            return (find(u, w) != x && find(u, w) >= 0 ? 1 : 0) + (find(v, w) != x && find(v, w) >= 0 ? 1 : 0);
+            if (!S.simple)
+              return (find(u, w) != x && find(u, w) >= 0 ? 1 : 0) + (find(v, w) != x && find(v, w) >= 0 ? 1 : 0);
+            // (of the two triangles at an edge the search above sees the one listed first)
+            const int ou = across(x, v, u, w), ov = across(x, u, v, w);
+            return (ou >= 0 && ou < x ? 1 : 0) + (ov >= 0 && ov < x ? 1 : 0);
           };
           keep = degree(t2, p, r) < degree(t1, q, r) + (code & 1);
         }
@@ -376,8 +420,10 @@ __global__ void k_rows_head(const PlanArgs a, const PartArgs p) {
       else if (n > 0) {
         // the beginning whose walk has the fewest steps; one strip around the
         // whole star, n + 2 steps, is found in two or three tries as a rule
+        Star S;
+        load_star(a, inc, n, S);
         auto steps_of = [&](int parts, int code) {
-          return walk_star(a, inc, n, parts, code, [](int, int, int, int, int, uint32_t) {});
+          return walk_star(S, parts, code, [](int, int, int, int, int, uint32_t) {});
         };
         int best = 0, least = steps_of(1, 0);
         for (int code = 1; code < min(6 * n, kStripTries) && least > n + 2; ++code) {
@@ -436,8 +482,10 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
         if (a.deg == 3) p.rec2[at] = make_uint4(0u, 0u, 0u, 0u);
       }
     };
-    if (n > 0 && n <= kMaxStar)
-      walk_star(a, inc, n, p.parts, p.own[t].z, [&](int part, int t, int r3, int p3, int q3, uint32_t flags) {
+    if (n > 0 && n <= kMaxStar) {
+      Star S;
+      load_star(a, inc, n, S);
+      walk_star(S, p.parts, p.own[t].z, [&](int part, int t, int r3, int p3, int q3, uint32_t flags) {
         while (at_part < part) {
           rest();
           ++at_part;
@@ -480,6 +528,7 @@ __global__ void k_rows_records(const PlanArgs a, const PartArgs p) {
         else p.rec[at] = w;
         if (a.deg == 3) p.rec2[at] = w2;
       });
+    }
     while (at_part < p.parts) {
       rest();
       ++at_part;
@@ -1329,14 +1378,17 @@ void build_part(const PlanArgs& a, PartArgs p, fe_form_s::RowsPlan::Part& part, 
   FE_CUDA(cudaStreamSynchronize(s));
   if (bad) return;
   const size_t nrec = (size_t)total * 32;
-  if (a.deg == 1) part.rec1.alloc(std::max<size_t>(1, nrec));
-  else part.rec.alloc(std::max<size_t>(1, nrec));
-  if (a.deg == 3 && p.kind != KIND_F) part.rec2.alloc(std::max<size_t>(1, nrec));
-  part.cell.alloc(std::max<size_t>(1, nrec));
-  p.rec = part.rec.p;
-  p.rec2 = part.rec2.p;
-  p.rec1 = part.rec1.p;
-  p.cell = part.cell.p;
+  // 16-byte records first, each array a multiple of 32 records long
+  const size_t one = a.deg == 1 ? sizeof(uint2) : (a.deg == 3 && p.kind != KIND_F ? 2 : 1) * sizeof(uint4);
+  part.mem.alloc(std::max<size_t>(1, nrec * (one + sizeof(int32_t))));
+  if (a.deg == 1) part.rec1 = reinterpret_cast<uint2*>(part.mem.p);
+  else part.rec = reinterpret_cast<uint4*>(part.mem.p);
+  if (a.deg == 3 && p.kind != KIND_F) part.rec2 = part.rec + nrec;
+  part.cell = reinterpret_cast<int32_t*>(part.mem.p + nrec * one);
+  p.rec = part.rec;
+  p.rec2 = part.rec2;
+  p.rec1 = part.rec1;
+  p.cell = part.cell;
   k_rows_records<<<blocks_for(p.ngroups * 32, 128), 128, 0, s>>>(a, p);
   FE_CUDA(cudaGetLastError());
   unsigned g = 0;
@@ -1396,11 +1448,10 @@ void build_rows_plan(fe_form_s& f, cudaStream_t s) {
     return;
   try {
     auto P = std::make_unique<fe_form_s::RowsPlan>();
-    // the temporaries in one allocation (a large one takes 0.3 ms, and as long to give back)
     size_t tb = 0;
     FE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr,
                                             (int32_t*)nullptr, (int)nR, 0, 32, s));
-    DevBuf<int32_t> work((tb + 3) / 4 + (size_t)C * V.k + 7 * (size_t)(nR + 1) + 8);
+    PlanScratch work(*f.ctx, (tb + 3) / 4 + (size_t)C * V.k + 7 * (size_t)(nR + 1) + 8, s);
     int32_t* next = work.p;
     auto take = [&](size_t n) {
       int32_t* q = next;
@@ -1514,11 +1565,11 @@ void launch_parts(const fe_form_s& f, WalkArgs a, cudaStream_t s) {
     a.ngroups = p.ngroups;
     a.own = p.own.p;
     a.steps = p.steps.p;
-    a.rec = p.rec.p;
-    a.rec2 = p.rec2.p;
+    a.rec = p.rec;
+    a.rec2 = p.rec2;
     a.own2 = p.own2.p;
-    a.rec1 = p.rec1.p;
-    a.cell = p.cell.p;
+    a.rec1 = p.rec1;
+    a.cell = p.cell;
     a.stride = p.stride;
     a.gaps = p.gaps ? 1 : 0;
   };
@@ -1547,9 +1598,9 @@ void launch_p3(const fe_form_s& f, WalkArgs a, cudaStream_t s) {
     a.own = p.own.p;
     a.own2 = p.own2.p;
     a.steps = p.steps.p;
-    a.rec = p.rec.p;
-    a.rec2 = p.rec2.p;
-    a.cell = p.cell.p;
+    a.rec = p.rec;
+    a.rec2 = p.rec2;
+    a.cell = p.cell;
     a.stride = p.stride;
     a.gaps = p.gaps ? 1 : 0;
     return (unsigned)p.ngroups;

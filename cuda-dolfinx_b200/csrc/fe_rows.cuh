@@ -149,6 +149,30 @@ void raise_smem(K kernel) {
   FE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemSm));
 }
 
+// The temporaries of a plan in one allocation: small ones from the context's
+// scratch pool, which keeps them for the next solve or plan (an allocation of
+// some MB takes 0.3 ms, and as long to give back), large ones on their own.
+struct PlanScratch {
+  static constexpr size_t kPooled = size_t(32) << 20;
+  int32_t* p = nullptr;
+  cudaStream_t s;
+  bool pooled;
+  PlanScratch(fe_context_s& ctx, size_t words, cudaStream_t st) : s(st), pooled(words * 4 <= kPooled) {
+    cudaMemPool_t pool = pooled ? scratch_pool(ctx) : nullptr;
+    const cudaError_t e = pooled ? cudaMallocFromPoolAsync((void**)&p, words * 4, pool, s) : cudaMalloc((void**)&p, words * 4);
+    if (e != cudaSuccess) {
+      p = nullptr;
+      (void)cudaGetLastError();
+      throw Error(FE_ERR_NOMEM, std::string("no memory for a plan's temporaries: ") + cudaGetErrorString(e));
+    }
+  }
+  PlanScratch(const PlanScratch&) = delete;
+  PlanScratch& operator=(const PlanScratch&) = delete;
+  ~PlanScratch() {
+    if (p) (void)(pooled ? cudaFreeAsync(p, s) : cudaFree(p));
+  }
+};
+
 void exclusive_scan(int32_t* v, int64_t n, cudaStream_t s) {
   size_t tb = 0;
   FE_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, v, v, (int)n, s));

@@ -476,11 +476,10 @@ void build_nodes_plan(fe_form_s& f, cudaStream_t s) {
     return;
   try {
     auto P = std::make_unique<fe_form_s::NodesPlan>();
-    // the temporaries in one allocation (a large one takes 0.3 ms, and as long to give back)
     size_t tb = 0;
     FE_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr,
                                             (int32_t*)nullptr, (int)nN, 0, 31, s));
-    DevBuf<int32_t> work((tb + 3) / 4 + (size_t)C * 10 + 7 * (size_t)(nN + 1) + 4);
+    PlanScratch work(*f.ctx, (tb + 3) / 4 + (size_t)C * 10 + 7 * (size_t)(nN + 1) + 4, s);
     int32_t* next = work.p;
     auto take = [&](size_t n) {
       int32_t* q = next;
