@@ -416,9 +416,11 @@ struct StreamScratch {
 // stop the host: at most kKeptRecords pairs are kept between solves
 struct HostRecords {
   fe_context_s& ctx;
-  Scalars* p = nullptr;  // two records
+  cudaStream_t s;
+  Scalars* p = nullptr;   // two records
+  bool in_flight = false; // a copy into them may be pending (an error left the solve)
   static constexpr size_t kKeptRecords = 16;
-  explicit HostRecords(fe_context_s& c) : ctx(c) {
+  HostRecords(fe_context_s& c, cudaStream_t st) : ctx(c), s(st) {
     {
       std::lock_guard<std::mutex> lock(ctx.host_mutex);
       if (!ctx.host_records.empty()) {
@@ -431,6 +433,7 @@ struct HostRecords {
   HostRecords(const HostRecords&) = delete;
   HostRecords& operator=(const HostRecords&) = delete;
   ~HostRecords() {
+    if (in_flight) (void)cudaStreamSynchronize(s);
     {
       std::lock_guard<std::mutex> lock(ctx.host_mutex);
       if (ctx.host_records.size() < kKeptRecords) {
@@ -542,6 +545,11 @@ template <int SUB>
 void run(const fe_sparsity_s& A, const double* val, const double* b, double* x, double rtol, int max_iter,
          int* iterations, double* rel_res, cudaStream_t s) {
   const int64_t n = A.num_rows;
+  // the host reads the stopping flag: refused before anything is captured (a
+  // copy into the records would outlive them in the graph)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  FE_CUDA(cudaStreamIsCapturing(s, &capture));
+  FE_REQUIRE(capture == cudaStreamCaptureStatusNone, "fe_pcg_solve reads its stopping flag and cannot be captured");
   const unsigned grid = (unsigned)(A.ctx->num_sms * 4);
   const unsigned grid_rows = (unsigned)(A.ctx->num_sms * 8);
   // stream-ordered scratch, released on every exit path (a launch or
@@ -557,7 +565,7 @@ void run(const fe_sparsity_s& A, const double* val, const double* b, double* x, 
   Scalars h{};
   h.tol2 = rtol * rtol;
   h.max_iter = max_iter;
-  HostRecords rec(*A.ctx);
+  HostRecords rec(*A.ctx, s);
   Event ev[2];
   cg_begin<SUB>(A, val, b, x, h, v, grid, grid_rows, s);
   // short iterations: a batch is always queued behind the one whose outcome
@@ -567,6 +575,7 @@ void run(const fe_sparsity_s& A, const double* val, const double* b, double* x, 
   int last = 0;
   for (int k = 0;; ++k) {
     cg_batch<SUB>(A, val, x, batch, v, grid, grid_rows, s);
+    rec.in_flight = true;
     FE_CUDA(cudaMemcpyAsync(rec.p + (k & 1), v.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
     FE_CUDA(cudaEventRecord(ev[k & 1].e, s));
     last = k;
@@ -576,6 +585,7 @@ void run(const fe_sparsity_s& A, const double* val, const double* b, double* x, 
     if (rec.p[seen & 1].done || (int64_t)seen * batch >= max_iter) break;
   }
   FE_CUDA(cudaEventSynchronize(ev[last & 1].e));  // the record is written until then
+  rec.in_flight = false;
   h = rec.p[last & 1];
   buf.release();
   *iterations = h.iter;
